@@ -168,12 +168,9 @@ struct XengineArgs {
     void *acc;                  // acc[b*n_freq + c] += (float2, or double2 if acc64)
     int acc64;
     int *err;
-    // plain X-engine: compute only the station-block pairs [pair_first,
-    // pair_first + pair_count) of its row-major enumeration (pair_count 0: all),
-    // or, with pair_list, the pair_count pairs it names
-    int pair_first;
-    int pair_count;
-    const int32_t *pair_list;
+    // plain X-engine: compute only these tiles (xengine_plain_tiles; nullptr: the
+    // whole matrix). Host memory, read during the launch call.
+    const std::vector<uint16_t> *tiles;
 };
 
 // fengine.cu
@@ -206,9 +203,11 @@ corr_status fengine_launch(int n_freq, const TwiddleTables &tw, const FengineArg
 
 // xengine.cu
 corr_status xengine_plain_launch(const XengineArgs &a, int num_sms, cudaStream_t stream);
-/// The plain X-engine's station-block pair holding baseline (j, k), j <= k: its
-/// index in the row-major enumeration of block pairs.
-int xengine_plain_block_pair(int n_station, int j, int k);
+/// The plain X-engine's tiles of 6 x 6 stations, each with the mask of its 3 x 3
+/// sub-blocks, that hold the given baselines (ascending indices of the row-major
+/// numbering j <= k; empty: all of them).
+void xengine_plain_tiles(int n_station, const std::vector<int32_t> &baselines,
+                         std::vector<uint16_t> *out);
 corr_status scale_launch(float2 *acc, size_t n, float s, cudaStream_t stream);
 /// acc[i] *= s in double precision over n complex128 values.
 corr_status scale64_launch(double2 *acc, size_t n, double s, cudaStream_t stream);
@@ -249,9 +248,7 @@ struct FxPlan {
     int fplan = 0;        // F-engine FFT radix plan
     int xmode = CORR_X_PLAIN_FP32;
     int acc64 = 0;        // rows are complex128 (CORRX_ACC_FP64) instead of complex64
-    int xpair_first = 0;  // plain X-engine: block pairs to compute (xpair_count 0: all)
-    int xpair_count = 0;
-    int32_t *d_xpair_list = nullptr;   // ... or the list of them (device memory)
+    std::vector<uint16_t> xtiles;   // plain X-engine: tiles to compute (empty: the whole matrix)
     int num_sms = 0;
     float2 *d_y = nullptr;
     int *d_err = nullptr;
@@ -262,7 +259,7 @@ corr_status fxplan_create(int device, int n_station, int n_freq, int max_frames,
                           FxPlan **out);
 void fxplan_destroy(FxPlan *p);
 corr_status fxplan_set_tiles(FxPlan *p, int ytile, int xct, int xkt, int fplan);
-/// The plain X-engine computes only the station-block pairs that hold the given
+/// The plain X-engine computes only the 3 x 3 station blocks that hold the given
 /// baselines (indices of the row-major numbering over the plan's stations); the
 /// other baselines of the row are left as they are. A device of a baseline-range
 /// split owns a contiguous range of them, one of pair covering a scattered set.

@@ -1,7 +1,7 @@
 // ptx.cuh -- thin inline-PTX wrappers used by the kernels (sm_103a).
 //
 // mbarrier + cp.async.bulk (TMA bulk copies) for the F-engine's input prefetch,
-// cp.async for the X-engines' staging, and the clock-bounded waits every spin
+// TMA tile loads for the X-engines, and the clock-bounded waits every spin
 // in this library goes through: a wait that runs out records a watchdog code in
 // a global flag and returns false instead of spinning for ever.
 
@@ -94,32 +94,37 @@ __device__ __forceinline__ void bulk_copy_g2s(void *dst, const void *src, uint32
         : "memory");
 }
 
+// 4-D TMA tile load global -> shared, completing on `bar`; `map` is a CUtensorMap in
+// kernel parameter space.
+__device__ __forceinline__ void tma_load_4d(void *dst, const void *map, int x, int y, int z,
+                                            int w, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_addr(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w),
+        "r"(smem_addr(bar))
+        : "memory");
+}
+
 // *dst += v, performed at L2, with no value returned to the thread.
 __device__ __forceinline__ void red_add_f64(double *dst, double v) {
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(gmem_addr(dst)), "d"(v) : "memory");
 }
 
-// 16-byte cp.async with zero fill when src_bytes == 0.
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, uint32_t src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)),
-                 "l"(gmem_addr(src)), "r"(src_bytes)
+// {dst[0], dst[1]} += v in FP32, performed at L2, with no value returned.
+__device__ __forceinline__ void red_add_f32x2(float2 *dst, float2 v) {
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(gmem_addr(dst)), "f"(v.x), "f"(v.y)
                  : "memory");
 }
 
-// Arrive on `bar` once every cp.async this thread issued so far has landed
-// (the arrival is not pre-counted: the barrier's count includes it).
-__device__ __forceinline__ void cp_async_mbar_arrive(uint64_t *bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar))
-                 : "memory");
-}
-
-__device__ __forceinline__ void cp_async_commit() {
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+// (double)x in integer arithmetic. This GPU converts (and computes) doubles at
+// 2 lanes per SM and cycle; a normal float only needs its exponent moved.
+__device__ __forceinline__ double widen(float x) {
+    const uint32_t b = __float_as_uint(x), m = b & 0x7fffffffu;
+    const bool normal = m - 0x00800000u < 0x7f000000u;
+    if (!normal && m != 0) return static_cast<double>(x);   // subnormal, infinite, NaN
+    const uint32_t hi = (b & 0x80000000u) | (normal ? (m >> 3) + 0x38000000u : 0u);
+    return __hiloint2double(static_cast<int>(hi), static_cast<int>(normal ? b << 29 : 0u));
 }
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {

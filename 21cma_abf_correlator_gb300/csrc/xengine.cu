@@ -5,170 +5,336 @@
 //     acc[b][c] += sum_f Y_j[f][c] * conj(Y_k[f][c])
 // with the reference's complex multiply-accumulate convention
 //     re += xr*yr + xi*yi,  im += xi*yr - xr*yi          (kernels.cu:243-245)
-// in FP32 and in that order (the product pair rounded, then added to the
-// accumulator), issued as packed FP32x2 instructions.
+// in FP32. Even and odd frames (and, for small problems, up to eight runs of them)
+// are summed apart, so a sum takes two fused multiply-adds per component and frame
+// and still rounds less than one long sum with a rounding per frame: relative RMS
+// against float64 at 24 inputs, n_freq 16384, 1024 frames 2.2e-7 (4.9e-7 with one
+// sum per visibility and the product pair rounded first).
 //
-// Shape: a CTA owns a tile of 32 channels (lane = channel) and a group of 4x4
-// station blocks (warp = block pair). Spectra for 2 to 12 frames of every
-// station in the tile are staged in shared memory by a 3-deep cp.async ring;
-// each thread keeps 16 complex accumulators in registers for the whole launch
-// and adds them into the row once at the end. Unlike the reference (one thread
-// per baseline, <= 1024 threads per block) the station-block tiling gives each
-// shared-memory load four multiply-accumulates.
+// Shape: a warp owns a 6 x 6 tile of the station matrix for 16 channels, one per
+// lane of each half warp; the half warps take even and odd frames. 72 sums and 24
+// operands per thread fit 128 registers, and a frame's 12 shared-memory loads feed
+// 144 multiply-adds: 24 bank cycles against 36 FP32 cycles, where a 4 x 4 tile's 8
+// loads per 64 take as long as its arithmetic. An 8 x 8 tile reads less still but
+// needs 168 registers (12 warps) and spilled around its loop; f32x2 instructions
+// want their operands broadcast and negated in pairs, one move per multiply-add.
+// Diagonal tiles leave out k < j, tiles of the last column the stations past the
+// end. Up to 15 such warps (every tile of a channel tile, then parts of the frames,
+// then channel tiles) and one that loads share a CTA; CTAs are persistent, and the
+// TMA ring runs on through their tiles, so that the end of one (two shuffles per
+// value, then reductions at L2) overlaps the loads of the next.
+//
+// Bound by FP32 issue: about 90 of the 128 lanes per SM and cycle in the loop
+// itself; the rest goes to scheduler imbalance (10 tiles on 4 schedulers at 24
+// inputs), stage boundaries and the last wave. Measured on one GB300, complex128
+// rows, before (4 x 4 tiles, 32 channels, cp.async, a CTA barrier per 2 to 12
+// frames) -> now:
+//   24 inputs, n_freq 16384, 1024 frames  1.90 -> 0.99 ms
+//   40 inputs, n_freq 16384,  512 frames  2.31 -> 1.48 ms
+//   64 inputs, n_freq  4096,  512 frames  1.94 -> 1.11 ms
+//   15 inputs, n_freq 12288,  301 frames  0.232 -> 0.135 ms
+//    4 inputs, n_freq  2048,  300 frames  0.093 -> 0.017 ms (64 one-warp CTAs before)
 
 #include <algorithm>
 #include <type_traits>
+#include <vector>
 
 #include "engine.h"
 #include "ptx.cuh"
+#include "tensor_map.h"
 
 namespace corrgb {
 namespace {
 
-constexpr int kXch = 32;     // channels per CTA, one per lane
-constexpr int kXstages = 3;  // cp.async ring depth
-// frames per pipeline stage: as many of 12, 8, 4, 2 as three stages fit in
-// shared memory (12 up to 24 padded stations, 8 up to 36, 4 up to 72, 2 up to
-// 144); fewer stages mean fewer CTA barriers
-constexpr int kXfsWidest = 12, kXfsWide = 8, kXfsNarrow = 4, kXfsTiny = 2;
-constexpr int kBlk = 4;      // stations per block
+constexpr int kXch = 16;      // channels of a warp's tile, one per lane of each half warp
+constexpr int kTile = 6;      // stations on each side of a warp's tile of the matrix
+constexpr int kSub = 3;       // stations on each side of a tile's four sub-blocks
+constexpr int kMaxWarps = 15; // summing warps per CTA; one more loads
+constexpr int kMaxSlots = 8;  // TMA ring depth, at most
+constexpr int kMaxParts = 8;  // runs of frames summed apart, at most
+constexpr int kSumElems = kTile * kSub * 32;   // float2 of a tile's sum
+constexpr int kMaxTiles = 253;   // 22 x 22 / 2 tiles of 128 stations
 
-__device__ __forceinline__ void decode_pair(int p, int nb, int *bj, int *bk) {
-    int j = 0;
-    while (p >= nb - j) {
-        p -= nb - j;
-        ++j;
-    }
-    *bj = j;
-    *bk = j + p;
-}
+// Which tiles a launch has: whole ones only; whole ones and, in the last column,
+// ones of at most kSub stations (n_station % kTile = 1 .. 3); any (some baselines
+// only). A kernel for each keeps its code, and so its instruction fetches, short.
+enum : int { kWhole = 0, kEdge = 1, kAny = 2 };
 
-template <int kXfs>
-__global__ void __launch_bounds__(1024, 1)
-    xengine_plain_kernel(const float2 *__restrict__ y, int y_frames, int ytile, int n_station,
-                         int npad, int n_freq, int frames, void *__restrict__ acc,
-                         int acc64, int pairs_per_cta, int pair_first, int n_pairs,
-                         const int32_t *__restrict__ pair_list) {
-    extern __shared__ __align__(16) float2 xs[];   // [stage][frame][npad][32]
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const int nthreads = blockDim.x;
-    const int c0 = blockIdx.y * kXch;
-    const int nb = npad / kBlk;
-    const int q = blockIdx.x * pairs_per_cta + warp;   // among the pairs computed
-    const bool active = q < n_pairs && warp < pairs_per_cta;
-    const int p = !active ? 0 : pair_list != nullptr ? pair_list[q] : pair_first + q;
-    int bj = 0, bk = 0;
-    if (active) decode_pair(p, nb, &bj, &bk);
+struct PlainParams {
+    int n_station;
+    int n_freq;
+    int frames;
+    int ytile;
+    int seg;              // frames per part (contiguous runs of the launch's frames, even)
+    int n_parts;
+    int tiles;            // CTA shape: tiles x part slots x channel tiles, a warp each
+    int slots_p;
+    int slots_c;
+    int fs;               // frames of each (channel tile, part) per ring slot, even
+    int slot_shift;       // ring slots: 1 << slot_shift
+    int n_tiles;          // tiles computed
+    int tile_groups;      // ceil(n_tiles / tiles)
+    int units;            // channel-tile groups x tile_groups
+    int sums_at;          // float2 before the tiles' sums in shared memory
+    void *acc;
+    int acc64;
+    int *err;
+    // J | K << 5 | sub-block mask << 10, groups of `tiles` one after the other (bit
+    // 2a + b of the mask: blocks of kSub stations 2J + a, 2K + b); mask 0: no tile
+    uint16_t tile[kMaxTiles + kMaxWarps];
+};
 
-    const int stage_elems = kXfs * npad * kXch;
-    const int chunks = stage_elems / 2;   // 16-byte pieces per stage
-    const int n_stages = (frames + kXfs - 1) / kXfs;
+// ROW: a run of frames in the ring holds [frame][station][16 channels] (ytile >= 16);
+// otherwise [spectra tile][frame][station][ytile], as the TMA box brings narrower tiles.
+// KIND: which tiles a launch has (kWhole, kEdge, kAny below).
+template <bool ROW, int KIND>
+__global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
+    xengine_plain_kernel(const __grid_constant__ CUtensorMap ymap,
+                         const __grid_constant__ PlainParams p) {
+    extern __shared__ __align__(128) float2 xs[];   // TMA ring, then the tiles' sums so far
+    __shared__ uint64_t full[kMaxSlots], empty[kMaxSlots];
+    __shared__ int s_abort;
+    __shared__ float2 zeros[kTile * kXch];   // a frame of one tile's stations that is not there
+    __shared__ int s_turn[kMaxWarps];   // per (channel tile, tile): parts summed
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n_warps = (blockDim.x >> 5) - 1;
+    const int N = p.n_station;
+    const volatile int *abort_flag = &s_abort;
+    const int slot_mask = (1 << p.slot_shift) - 1;
 
-    // Every thread copies the same two channels (blockDim is a multiple of 16):
-    // piece `part` of each (frame, station) row of the stage.
-    const int part = threadIdx.x & 15;
-    const int cq = c0 + part * 2;
-    const float2 *ybase = y + y_index(cq, 0, 0, n_station, y_frames, ytile);
-    auto load_stage = [&](int s) {
-        float2 *dst = xs + (s % kXstages) * stage_elems;
-        const int f0 = s * kXfs;
-        for (int q = threadIdx.x; q < chunks; q += nthreads) {
-            const int row = q >> 4;                  // frame*npad + station
-            const int fi = row / npad;
-            const int st = row - fi * npad;
-            const int f = f0 + fi;
-            const bool ok = (st < n_station) && (f < frames);
-            // two channels per 16-byte piece, inside one channel tile
-            const float2 *src =
-                ok ? ybase + (static_cast<size_t>(f) * n_station + st) * ytile : y;
-            cp_async16(dst + row * kXch + part * 2, src, ok ? 16u : 0u);
+    if (tid == 0) {
+        for (int s = 0; s <= slot_mask; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], n_warps);
         }
-    };
-
-    float2 a[kBlk][kBlk];
-#pragma unroll
-    for (int i = 0; i < kBlk; ++i)
-#pragma unroll
-        for (int l = 0; l < kBlk; ++l) a[i][l] = make_float2(0.f, 0.f);
-
-#pragma unroll
-    for (int s = 0; s < kXstages - 1; ++s) {
-        if (s < n_stages) load_stage(s);
-        cp_async_commit();
+        s_abort = 0;
+        fence_mbar_init();
     }
-    for (int s = 0; s < n_stages; ++s) {
-        cp_async_wait<kXstages - 2>();
-        __syncthreads();
-        if (s + kXstages - 1 < n_stages) load_stage(s + kXstages - 1);
-        cp_async_commit();
-        if (active) {
-            const float2 *st = xs + (s % kXstages) * stage_elems;
-            // A warp whose two blocks are the same keeps only j <= k: it loads
-            // one block and skips the pairs below the diagonal (uniform per warp).
-            auto stage = [&](auto diag) {
-                constexpr bool DIAG = decltype(diag)::value;
-#pragma unroll
-                for (int fi = 0; fi < kXfs; ++fi) {
-                    const float2 *fr = st + fi * npad * kXch + lane;
-                    float2 xj[kBlk], xk[kBlk];
-#pragma unroll
-                    for (int i = 0; i < kBlk; ++i) {
-                        xj[i] = fr[(bj * kBlk + i) * kXch];
-                        xk[i] = DIAG ? xj[i] : fr[(bk * kBlk + i) * kXch];
+    if (tid < kMaxWarps) s_turn[tid] = 0;
+    for (int i = tid; i < kTile * kXch; i += blockDim.x) zeros[i] = make_float2(0.f, 0.f);
+    __syncthreads();
+
+    // The CTA walks units (a tile group of a group of channel tiles), each in
+    // n_parts / slots_p rounds, each round in stages of fs frames per part; the
+    // ring of stages runs on through all of them.
+    const int rounds = p.n_parts / p.slots_p;
+    auto part_frames = [&](int t) { return max(0, min(p.seg, p.frames - t * p.seg)); };
+    auto round_stages = [&](int r) {   // by its first, longest part
+        return (part_frames(r * p.slots_p) + p.fs - 1) / p.fs;
+    };
+    const int run_elems = p.fs * N * kXch;
+    const int slot_elems = p.slots_c * p.slots_p * run_elems;
+
+    if (warp == n_warps) {
+        // ------------------------------ loader ------------------------------
+        if (lane == 0) {
+            int n = 0;   // stages issued
+            bool ok = true;
+            for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
+                const int ct0 = u / p.tile_groups * p.slots_c;
+                const int n_ct = min(p.slots_c, p.n_freq / kXch - ct0);
+                for (int r = 0; r < rounds && ok; ++r) {
+                    const int stages = round_stages(r);
+                    for (int s = 0; s < stages; ++s, ++n) {
+                        const int slot = n & slot_mask;
+                        if (n > slot_mask &&
+                            !mbar_wait_bounded(&empty[slot],
+                                               static_cast<uint32_t>((n >> p.slot_shift) - 1) & 1u,
+                                               p.err, kErrXengineMmaTimeout, abort_flag)) {
+                            s_abort = 1;
+                            ok = false;
+                            break;
+                        }
+                        mbar_arrive_expect_tx(
+                            &full[slot],
+                            static_cast<uint32_t>(n_ct * p.slots_p * run_elems * sizeof(float2)));
+                        // frames past the launch's arrive as zeros, those past their
+                        // part are not used
+                        float2 *dst = xs + slot * slot_elems;
+                        for (int c = 0; c < n_ct; ++c) {
+                            const int ch = (ct0 + c) * kXch;
+                            for (int i = 0; i < p.slots_p; ++i, dst += run_elems)
+                                tma_load_4d(dst, &ymap, ch % p.ytile, 0,
+                                            (r * p.slots_p + i) * p.seg + s * p.fs, ch / p.ytile,
+                                            &full[slot]);
+                        }
                     }
-                    // a += xj * conj(xk) in the reference's rounding order (the
-                    // pair's product, then one add to the accumulator), packed:
-                    //   t = (xj.x, xj.y) * (xk.x, xk.x)
-                    //   t = (xj.y, -xj.x) * (xk.y, xk.y) + t
-                    //   (re, im) += t
-                    // the swapped and broadcast operands built once per station
-                    float2 xjs[kBlk];
+                }
+            }
+            // An aborted CTA lets every load in flight land before it exits. (One
+            // that ran through has read them all.)
+            if (!ok)
+                for (int s = 0; s <= slot_mask; ++s) {
+                    const uint32_t n_s = static_cast<uint32_t>(n + slot_mask - s) >> p.slot_shift;
+                    if (n_s > 0) mbar_wait_bounded(&full[s], (n_s - 1) & 1u, nullptr, 0);
+                }
+        }
+        return;
+    }
+
+    // ------------------------------- sums -------------------------------
+    // this warp's place in the CTA: tile, part slot, channel tile
+    const int wt = warp % p.tiles, wp = (warp / p.tiles) % p.slots_p;
+    const int wc = warp / (p.tiles * p.slots_p);
+    volatile int *turn = &s_turn[wc * p.tiles + wt];   // the part to come
+    float2 *const so_far = xs + p.sums_at + (wc * p.tiles + wt) * kSumElems + lane;
+    const int rs = ROW ? kXch : p.ytile;   // float2 between stations of a run
+    const int half = lane >> 4, ch = lane & 15;   // half warp: even or odd frames of the part
+    const int lane_off = ROW ? ch : (ch / rs) * (p.fs * N * rs) + ch % rs;
+    int used = 0;   // stages of the ring read
+
+    for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
+        const int ct = u / p.tile_groups * p.slots_c + wc;
+        const int entry = ct < p.n_freq / kXch ? p.tile[u % p.tile_groups * p.tiles + wt] : 0;
+        const int J = entry & 31, K = (entry >> 5) & 31, sub = entry >> 10;
+        for (int r = 0; r < rounds; ++r) {
+            const int t = r * p.slots_p + wp;
+            const int n_mine = part_frames(t);
+            // visibilities of stations j = 6J + i and k = 6K + l
+            float re[kTile][kTile], im[kTile][kTile];
 #pragma unroll
-                    for (int i = 0; i < kBlk; ++i) xjs[i] = make_float2(xj[i].y, -xj[i].x);
+            for (int i = 0; i < kTile; ++i)
 #pragma unroll
-                    for (int l = 0; l < kBlk; ++l) {
-                        const float2 kx = make_float2(xk[l].x, xk[l].x);
-                        const float2 ky = make_float2(xk[l].y, xk[l].y);
-#pragma unroll
-                        for (int i = 0; i < kBlk; ++i)
-                            if (!DIAG || i <= l)
-                                a[i][l] = cadd(a[i][l], fma2(xjs[i], ky, mul2(xj[i], kx)));
+                for (int l = 0; l < kTile; ++l) re[i][l] = im[i][l] = 0.f;
+
+            // The round's frames, two a step, one per half warp: the sub-blocks of
+            // `mask`; on a tile of the diagonal (DIAG) the pairs k < j are left out.
+            auto sum_frames = [&](auto mask_tag, auto diag_tag, int mask_arg) {
+                constexpr int MASK = decltype(mask_tag)::value;
+                constexpr bool DIAG = decltype(diag_tag)::value;
+                const int mask = MASK != 0 ? MASK : mask_arg;
+                const float2 *const run = xs + (wc * p.slots_p + wp) * run_elems + lane_off +
+                                          (half * N + J * kTile) * rs;
+                const int to_k = (K - J) * kTile * rs;
+                const int step = 2 * N * rs;
+                int n_left = n_mine;
+                for (int s = round_stages(r); s > 0; --s, n_left -= p.fs, ++used) {
+                    const int slot = used & slot_mask;
+                    if (!mbar_wait_bounded(&full[slot],
+                                           static_cast<uint32_t>(used >> p.slot_shift) & 1u, p.err,
+                                           kErrXengineMmaTimeout, abort_flag)) {
+                        s_abort = 1;
+                        return;
                     }
+                    const float2 *xj = run + slot * slot_elems;
+                    const int nf = MASK == 0 && KIND != kAny ? 0 : min(p.fs, n_left);
+#pragma unroll 1
+                    for (int f = 0; f < nf; f += 2, xj += step) {
+                        // the odd frame of a last pair, which is not there, counts as zeros
+                        const float2 *yk = f + half < nf ? xj + to_k : zeros + lane_off;
+                        constexpr int NY = MASK == 0x5 || MASK == 0x1 ? kSub : kTile;
+                        constexpr int NX = MASK == 0x1 ? kSub : kTile;
+                        float2 x[kTile], y[kTile];
+#pragma unroll
+                        for (int l = 0; l < NY; ++l) y[l] = yk[l * rs];
+#pragma unroll
+                        for (int i = 0; i < NX; ++i) x[i] = DIAG ? y[i] : xj[i * rs];
+                        // j = 6J + i against k = 6K + l, l0 <= l < l1
+                        auto mac = [&](int i, int l0, int l1) {
+#pragma unroll
+                            for (int l = l0; l < l1; ++l) {
+                                re[i][l] = fmaf(x[i].x, y[l].x, re[i][l]);
+                                im[i][l] = fmaf(x[i].y, y[l].x, im[i][l]);
+                            }
+#pragma unroll
+                            for (int l = l0; l < l1; ++l) {
+                                re[i][l] = fmaf(x[i].y, y[l].y, re[i][l]);
+                                im[i][l] = fmaf(-x[i].x, y[l].y, im[i][l]);
+                            }
+                        };
+                        if constexpr (MASK != 0) {
+#pragma unroll
+                            for (int i = 0; i < NX; ++i) mac(i, DIAG ? i : 0, NY);
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                                if ((mask >> q) & 1) {
+#pragma unroll
+                                    for (int i = 0; i < kSub; ++i)
+                                        mac(q / 2 * kSub + i, q % 2 * kSub, q % 2 * kSub + kSub);
+                                }
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&empty[slot]);
                 }
             };
-            if (bj == bk)
-                stage(std::true_type{});
-            else
-                stage(std::false_type{});
-        }
-    }
-    cp_async_wait<0>();
+            using std::integral_constant;
+            if (sub == 0xf) {
+                sum_frames(integral_constant<int, 0xf>{}, std::false_type{}, 0);
+            } else if (sub == 0xb && J == K) {   // a whole tile of the diagonal
+                sum_frames(integral_constant<int, 0xb>{}, std::true_type{}, 0);
+            } else if (KIND == kAny) {
+                sum_frames(integral_constant<int, 0>{}, std::false_type{}, sub);
+            } else if (KIND == kEdge && sub == 0x5) {   // the last column, of 1 to 3 stations
+                sum_frames(integral_constant<int, 0x5>{}, std::false_type{}, 0);
+            } else if (KIND == kEdge && sub == 0x1) {   // and its diagonal tile
+                sum_frames(integral_constant<int, 0x1>{}, std::true_type{}, 0);
+            } else {   // no tile: the slots only pass
+                sum_frames(integral_constant<int, 0>{}, std::false_type{}, 0);
+            }
+            if (s_abort) return;
+            if (sub == 0) continue;
 
-    if (!active) return;
-    const int c = c0 + lane;
-#pragma unroll
-    for (int i = 0; i < kBlk; ++i) {
-        const int j = bj * kBlk + i;
-#pragma unroll
-        for (int l = 0; l < kBlk; ++l) {
-            const int k = bk * kBlk + l;
-            if (j <= k && k < n_station) {
-                const int b = j * n_station - j * (j - 1) / 2 + (k - j);
-                const size_t at = static_cast<size_t>(b) * n_freq + c;
-                if (acc64) {   // complex128 row: the launch's FP32 sum added in double
-                    double2 *dst = static_cast<double2 *>(acc) + at;
-                    double2 v = *dst;
-                    v.x += a[i][l].x;
-                    v.y += a[i][l].y;
-                    *dst = v;
-                } else {
-                    float2 *dst = static_cast<float2 *>(acc) + at;
-                    float2 v = *dst;
-                    v.x += a[i][l].x;
-                    v.y += a[i][l].y;
-                    *dst = v;
+            // The half warps' sums together (even + odd frames), each half warp
+            // keeping three of the six rows. Then part after part (turn): each adds
+            // to the sum so far of its tile, in shared memory, and the last one adds
+            // the total to the row, as reductions at L2 (the launch's only ones to
+            // those values), so that the result does not depend on the warps' timing.
+            if (p.n_parts > 1) {   // part 0: until the tile before is through
+                const long long t0 = clock64();
+                bool mine = true;
+                while (*turn != t) {
+                    if (s_abort || clock64() - t0 > kWaitBudgetCycles) {
+                        mine = false;
+                        break;
+                    }
                 }
+                if (!__all_sync(0xffffffffu, mine)) {
+                    if (p.err != nullptr && s_abort == 0) atomicExch(p.err, kErrXengineMmaTimeout);
+                    s_abort = 1;
+                    return;
+                }
+                __threadfence_block();
+            }
+            const size_t c = static_cast<size_t>(ct) * kXch + ch;
+#pragma unroll
+            for (int i3 = 0; i3 < kSub; ++i3) {
+                const int j = J * kTile + kSub * half + i3;
+                // where baseline (j, 0) of a full square would be
+                const size_t row = static_cast<size_t>(j * N - j * (j + 1) / 2) * p.n_freq + c;
+#pragma unroll
+                for (int l = 0; l < kTile; ++l) {
+                    const float gr = half ? re[i3][l] : re[kSub + i3][l];   // the other's
+                    const float gi = half ? im[i3][l] : im[kSub + i3][l];
+                    const float ar = __shfl_xor_sync(0xffffffffu, gr, 16);
+                    const float ai = __shfl_xor_sync(0xffffffffu, gi, 16);
+                    const float mr = half ? re[kSub + i3][l] : re[i3][l];
+                    const float mi = half ? im[kSub + i3][l] : im[i3][l];
+                    float2 v = make_float2(mr + ar, mi + ai);
+                    const int e = (i3 * kTile + l) * 32;
+                    if (t > 0) v = cadd(so_far[e], v);
+                    if (t < p.n_parts - 1) {
+                        so_far[e] = v;
+                        continue;
+                    }
+                    const int k = K * kTile + l;
+                    if (j <= k && k < N && ((sub >> (2 * half + l / kSub)) & 1)) {
+                        const size_t at = row + static_cast<size_t>(k) * p.n_freq;
+                        if (p.acc64) {   // complex128 row: the FP32 sums added in double
+                            double *dst = static_cast<double *>(p.acc) + 2 * at;
+                            red_add_f64(dst, widen(v.x));
+                            red_add_f64(dst + 1, widen(v.y));
+                        } else {
+                            red_add_f32x2(static_cast<float2 *>(p.acc) + at, v);
+                        }
+                    }
+                }
+            }
+            if (p.n_parts > 1) {
+                __threadfence_block();
+                __syncwarp();
+                if (lane == 0) *turn = (t + 1) % p.n_parts;
             }
         }
     }
@@ -271,66 +437,190 @@ corr_status watchdog_selftest_launch(int *err, long long budget_cycles, cudaStre
     return cuda_check(cudaGetLastError(), "watchdog_selftest_kernel launch");
 }
 
-corr_status xengine_plain_launch(const XengineArgs &a, int num_sms, cudaStream_t stream) {
-    (void)num_sms;
-    if (a.frames <= 0) return CORR_OK;
-    const int npad = (a.n_station + kBlk - 1) / kBlk * kBlk;
-    const int nb = npad / kBlk;
-    const int all_pairs = nb * (nb + 1) / 2;
-    const bool list = a.pair_list != nullptr && a.pair_count > 0 && a.pair_count <= all_pairs;
-    const bool part = list || (a.pair_count > 0 && a.pair_first >= 0 &&
-                               a.pair_first + a.pair_count <= all_pairs);
-    const int pair_first = part && !list ? a.pair_first : 0;
-    const int n_pairs = part ? a.pair_count : all_pairs;
-    const int groups = (n_pairs + 31) / 32;
-    const int per_cta = (n_pairs + groups - 1) / groups;
-    const size_t per_frame = static_cast<size_t>(kXstages) * npad * kXch * sizeof(float2);
-    // Deeper stages mean fewer CTA barriers, but a CTA of few warps (as when only
-    // some block pairs are computed) needs others beside it on its SM: take the
-    // deepest stages among those that give an SM the most warps, up to 16.
-    int fs = 0, best = -1;
-    for (int f : {kXfsWidest, kXfsWide, kXfsNarrow, kXfsTiny}) {
-        const size_t bytes = per_frame * f;
-        if (bytes > 227 * 1024) continue;
-        const int warps = std::min(16, static_cast<int>((227 * 1024) / bytes) * per_cta);
-        if (warps > best) {
-            best = warps;
-            fs = f;
+// Parts of a launch: its frames in contiguous runs, summed apart and then added up
+// in order. One, or more where the channels alone leave warps idle and a part
+// keeps 16 frames. A function of n_freq and frames alone, never of the station
+// count or of the baselines computed: devices that hold different stations of one
+// run sum the same sets of frames and agree to the bit. (Even and odd frames are
+// summed apart too, so that no sum runs over more than half of the frames: its
+// two roundings per frame then leave less error than one rounding per frame of a
+// sum over all of them.)
+static int plain_parts(int n_freq, int frames) {
+    int h = 1;
+    while (h < kMaxParts && n_freq / kXch * h < 152 * 12 && frames / (2 * h) >= 16) h *= 2;
+    return h;
+}
+
+void xengine_plain_tiles(int n_station, const std::vector<int32_t> &baselines,
+                         std::vector<uint16_t> *out) {
+    const int nb = (n_station + kTile - 1) / kTile;
+    std::vector<int> mask(static_cast<size_t>(nb) * nb, 0);
+    auto mark = [&](int j, int k) {
+        mask[static_cast<size_t>(j / kTile) * nb + k / kTile] |=
+            1 << (2 * (j / kSub % 2) + k / kSub % 2);
+    };
+    int b = 0;
+    size_t next = 0;   // into the (ascending) baselines
+    for (int j = 0; j < n_station; ++j)
+        for (int k = j; k < n_station; ++k, ++b) {
+            if (baselines.empty()) {
+                mark(j, k);
+            } else if (next < baselines.size() && baselines[next] == b) {
+                mark(j, k);
+                ++next;
+            }
+        }
+    out->clear();
+    for (int J = 0; J < nb; ++J)
+        for (int K = J; K < nb; ++K)
+            if (const int m = mask[static_cast<size_t>(J) * nb + K])
+                out->push_back(static_cast<uint16_t>(J | (K << 5) | (m << 10)));
+}
+
+// Multiply-accumulates per pair of frames of a tile entry, about.
+static int tile_weight(uint16_t e) {
+    const bool diag = (e & 31) == ((e >> 5) & 31);
+    int w = 0;
+    for (int q = 0; q < 4; ++q)
+        if ((e >> (10 + q)) & 1) w += diag && q != 1 ? 6 : 9;
+    return w + 3;   // and the loads
+}
+
+// Deal the tiles to the groups, and inside a group to the warps, so that the SM's
+// four schedulers (warp % 4) get shares as equal as may be: heaviest first, each
+// to the group, then to the place, where the most loaded scheduler has least.
+static void place_tiles(std::vector<uint16_t> tiles, PlainParams *p) {
+    std::sort(tiles.begin(), tiles.end(), [](uint16_t a, uint16_t b) {
+        const int wa = tile_weight(a), wb = tile_weight(b);
+        return wa != wb ? wa > wb : a < b;
+    });
+    std::vector<std::vector<uint16_t>> group(static_cast<size_t>(p->tile_groups));
+    std::vector<int> load(group.size(), 0);
+    for (uint16_t e : tiles) {
+        size_t g = group.size();
+        for (size_t i = 0; i < group.size(); ++i)
+            if (static_cast<int>(group[i].size()) < p->tiles && (g == group.size() || load[i] < load[g]))
+                g = i;
+        group[g].push_back(e);
+        load[g] += tile_weight(e);
+    }
+    const int copies = p->slots_p * p->slots_c;
+    for (size_t g = 0; g < group.size(); ++g) {
+        uint16_t *slot = p->tile + g * p->tiles;
+        std::fill(slot, slot + p->tiles, uint16_t(0));
+        int busy[4] = {0, 0, 0, 0};
+        for (uint16_t e : group[g]) {
+            int best = -1, best_peak = 0;
+            for (int at = 0; at < p->tiles; ++at) {
+                if (slot[at] != 0) continue;
+                int b[4] = {busy[0], busy[1], busy[2], busy[3]};
+                for (int c = 0; c < copies; ++c) b[(at + c * p->tiles) % 4] += tile_weight(e);
+                int sq = 0;
+                for (int v : b) sq += v * v;
+                if (best < 0 || sq < best_peak) {
+                    best = at;
+                    best_peak = sq;
+                }
+            }
+            slot[best] = e;
+            for (int c = 0; c < copies; ++c) busy[(best + c * p->tiles) % 4] += tile_weight(e);
         }
     }
-    if (fs == 0 || per_frame * fs > 227 * 1024)
-        return failf(CORR_ERR_ARG, "plain X-engine: %d stations do not fit in shared memory",
-                     a.n_station);
-    const size_t smem = per_frame * fs;
+}
+
+corr_status xengine_plain_launch(const XengineArgs &a, int num_sms, cudaStream_t stream) {
+    if (a.frames <= 0) return CORR_OK;
+    const int N = a.n_station;
+    std::vector<uint16_t> tiles;
+    if (a.tiles != nullptr)
+        tiles = *a.tiles;
+    else
+        xengine_plain_tiles(N, {}, &tiles);
+    PlainParams p{};
+    p.n_tiles = static_cast<int>(tiles.size());
+    if (p.n_tiles == 0) return CORR_OK;
+    const int n_ct = a.n_freq / kXch;
+    p.n_parts = plain_parts(a.n_freq, a.frames);
+    p.seg = ((a.frames + p.n_parts - 1) / p.n_parts + 1) / 2 * 2;
+    // CTA shape: every tile of a channel tile if they fit, in tile groups (that
+    // read the same spectra) otherwise; then parts side by side; then channel
+    // tiles, as long as each SM still gets a CTA.
+    p.tile_groups = (p.n_tiles + kMaxWarps - 1) / kMaxWarps;
+    p.tiles = (p.n_tiles + p.tile_groups - 1) / p.tile_groups;
+    p.slots_p = 1;
+    while (p.slots_p < p.n_parts && p.tiles * p.slots_p * 2 <= kMaxWarps) p.slots_p *= 2;
+    p.slots_c = 1;
+    while (p.tiles * p.slots_p * (p.slots_c + 1) <= kMaxWarps &&
+           (n_ct + p.slots_c) / (p.slots_c + 1) * p.tile_groups >= num_sms)
+        ++p.slots_c;
+    p.units = (n_ct + p.slots_c - 1) / p.slots_c * p.tile_groups;
+    place_tiles(tiles, &p);
+    // Ring: four slots (eight if they are small), each as long as fits; rows past
+    // the last station are read (and dropped) by the last tile, hence the pad.
+    const size_t per_pair = static_cast<size_t>(2) * N * kXch * sizeof(float2) * p.slots_p * p.slots_c;
+    const size_t pad = static_cast<size_t>(kTile) * kXch * sizeof(float2);
+    const int warps = p.tiles * p.slots_p * p.slots_c + 1;
+    const int per_sm = std::max(1, (kMaxWarps + 1) / warps);
+    const size_t sums = p.n_parts > 1 ? p.tiles * p.slots_c * kSumElems * sizeof(float2) : 0;
+    const size_t budget = static_cast<size_t>(224 * 1024) / per_sm - 2048 - pad - sums;
+    p.slot_shift = 8 * 16 * per_pair <= budget ? 3 : 2;
+    if ((per_pair << p.slot_shift) > budget)
+        return failf(CORR_ERR_ARG, "plain X-engine: %d stations do not fit in shared memory", N);
+    p.fs = 2 * static_cast<int>(std::min<size_t>(16, (budget >> p.slot_shift) / per_pair));
+    const size_t ring = ((per_pair * (p.fs / 2)) << p.slot_shift) + pad;
+    p.sums_at = static_cast<int>(ring / sizeof(float2));
+    const size_t smem = ring + sums;
+    p.n_station = N;
+    p.n_freq = a.n_freq;
+    p.frames = a.frames;
+    p.ytile = a.ytile;
+    p.acc = a.acc;
+    p.acc64 = a.acc64;
+    p.err = a.err;
+
+    EncodeTiledFn enc = encode_tiled();
+    if (enc == nullptr)
+        return fail(CORR_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    // Spectra as (channel within its tile, station, frame, tile), 8 bytes a bin.
+    const cuuint32_t box_c = static_cast<cuuint32_t>(std::min(a.ytile, kXch));
+    const cuuint64_t row = static_cast<cuuint64_t>(a.ytile) * sizeof(float2);
+    CUtensorMap map;
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    const cuuint64_t dims[4] = {static_cast<cuuint64_t>(a.ytile), static_cast<cuuint64_t>(N),
+                                static_cast<cuuint64_t>(a.frames),
+                                static_cast<cuuint64_t>(a.n_freq / a.ytile)};
+    const cuuint64_t strides[3] = {row, row * N, row * N * a.y_frames};
+    const cuuint32_t box[4] = {box_c, static_cast<cuuint32_t>(N), static_cast<cuuint32_t>(p.fs),
+                               kXch / box_c};
+    const CUresult cr =
+        enc(&map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, const_cast<float2 *>(a.y), dims, strides,
+            box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS)
+        return failf(CORR_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", static_cast<int>(cr));
+
+    using Kernel = void (*)(CUtensorMap, PlainParams);
+    static constexpr Kernel kernels[6] = {
+        xengine_plain_kernel<true, kWhole>, xengine_plain_kernel<true, kEdge>,
+        xengine_plain_kernel<true, kAny>,   xengine_plain_kernel<false, kWhole>,
+        xengine_plain_kernel<false, kEdge>, xengine_plain_kernel<false, kAny>};
     static PerDevice setup;   // the shared-memory limit is a per-device setting
     corr_status st = setup.run([](int) {
-        for (auto k : {xengine_plain_kernel<kXfsWidest>, xengine_plain_kernel<kXfsWide>,
-                       xengine_plain_kernel<kXfsNarrow>, xengine_plain_kernel<kXfsTiny>}) {
+        for (auto k : kernels) {
             corr_status s2 =
                 cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                227 * 1024),
+                                                224 * 1024),
                            "cudaFuncSetAttribute(xengine_plain)");
             if (s2 != CORR_OK) return s2;
         }
         return CORR_OK;
     });
     if (st != CORR_OK) return st;
-    dim3 grid(groups, a.n_freq / kXch);
-    auto k = fs == kXfsWidest ? xengine_plain_kernel<kXfsWidest>
-           : fs == kXfsWide   ? xengine_plain_kernel<kXfsWide>
-           : fs == kXfsNarrow ? xengine_plain_kernel<kXfsNarrow>
-                              : xengine_plain_kernel<kXfsTiny>;
-    k<<<grid, per_cta * 32, smem, stream>>>(a.y, a.y_frames, a.ytile, a.n_station, npad,
-                                            a.n_freq, a.frames, a.acc, a.acc64, per_cta,
-                                            pair_first, n_pairs, list ? a.pair_list : nullptr);
+    const int grid = std::min(p.units, std::max(1, num_sms) * per_sm);
+    const int kind = a.tiles != nullptr ? kAny : (N - 1) % kTile < kSub ? kEdge : kWhole;
+    const Kernel kernel = kernels[(a.ytile >= kXch ? 0 : 3) + kind];
+    kernel<<<grid, warps * 32, smem, stream>>>(map, p);
     return cuda_check(cudaGetLastError(), "xengine_plain_kernel launch");
-}
-
-int xengine_plain_block_pair(int n_station, int j, int k) {
-    const int nb = (n_station + kBlk - 1) / kBlk;
-    const int bj = j / kBlk, bk = k / kBlk;
-    // block pairs (bj, bk), bj <= bk, row-major
-    return bj * nb - bj * (bj - 1) / 2 + (bk - bj);
 }
 
 corr_status scale_launch(float2 *acc, size_t n, float s, cudaStream_t stream) {

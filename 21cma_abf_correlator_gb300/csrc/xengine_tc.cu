@@ -68,6 +68,7 @@
 
 #include "engine.h"
 #include "ptx.cuh"
+#include "tensor_map.h"
 
 namespace corrgb {
 namespace {
@@ -265,17 +266,6 @@ __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t *r) {
 
 __device__ __forceinline__ void tmem_ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// 4-D TMA tile load global -> shared, completing on `bar`.
-__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int x, int y, int z,
-                                            int w, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-        "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_addr(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w),
-        "r"(smem_addr(bar))
-        : "memory");
 }
 
 struct TcParams {
@@ -797,12 +787,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 }
 
-// cuTensorMapEncodeTiled from the driver, looked up once through the runtime
-// (no link-time dependency on libcuda).
-using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                                   const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                   const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+} // namespace
 
 EncodeTiledFn encode_tiled() {
     static EncodeTiledFn fn = nullptr;
@@ -819,8 +804,6 @@ EncodeTiledFn encode_tiled() {
     });
     return fn;
 }
-
-} // namespace
 
 bool xengine_tc_shape_ok(int n_station, bool split, int ct, int kt) {
     return make_geom(n_station, split, ct, kt).ok;
