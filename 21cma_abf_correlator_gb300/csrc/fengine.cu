@@ -32,7 +32,8 @@
 #include "fengine_impl.cuh"
 
 // This file: the host side (twiddle tables, plans, dispatch by length) and the
-// kernels of n_freq 512 .. 8192; fengine_impl.cuh holds the kernel templates.
+// kernels of n_freq 512 .. 2048 and, for few frames, of 4096 .. 8192; fengine_impl.cuh
+// holds the kernel templates, fengine_rows.cuh those of 4096 .. 16384.
 
 namespace corrgb {
 
@@ -103,11 +104,27 @@ corr_status fengine_launch(int n_freq, const TwiddleTables &tw, const FengineArg
     case 512: return launch_size<512>(a, tw, num_sms, stream);
     case 1024: return launch_size<1024>(a, tw, num_sms, stream);
     case 2048: return launch_size<2048>(a, tw, num_sms, stream);
-    case 4096: return launch_size<4096>(a, tw, num_sms, stream);
-    case 6144: return launch_size<6144>(a, tw, num_sms, stream);
-    case 8192: return launch_size<8192>(a, tw, num_sms, stream);
-    case 10240: case 12288: case 14336: case 16384:
-        return fengine_launch_large(n_freq, tw, a, num_sms, stream);
+    // The kernel of fengine_rows.cuh starts 2 us slower (its tensor-memory tables) and
+    // is faster per frame. 24 stations, FP16 output, old / rows: n_freq 4096 4 frames
+    // 6.9 / 9.0 us, 64 frames 18.9 / 21.1, 512 frames 115.2 / 109.8; n_freq 8192 4
+    // frames 8.5 / 10.7, 1024 frames 483 / 433. (From 10240 up it is the faster one
+    // from a few frames on: 12288 4 frames 12.7 / 13.0, 1024 frames 1115 / 900.) By
+    // frames alone, so that devices holding different stations take the same one.
+    case 4096:
+        if (a.frames < 256) return launch_size<4096>(a, tw, num_sms, stream);
+        return fengine_launch_rows_c(n_freq, tw, a, num_sms, stream);
+    case 6144:
+        if (a.frames < 64) return launch_size<6144>(a, tw, num_sms, stream);
+        return fengine_launch_rows_c(n_freq, tw, a, num_sms, stream);
+    case 8192:
+        if (a.frames < 64) return launch_size<8192>(a, tw, num_sms, stream);
+        return fengine_launch_rows_c(n_freq, tw, a, num_sms, stream);
+    case 10240: case 12288: return fengine_launch_rows_b(n_freq, tw, a, num_sms, stream);
+    case 14336: return fengine_launch_rows_a(n_freq, tw, a, num_sms, stream);
+    case 16384:
+        if (a.fplan == 1) return fengine_launch_plan1(tw, a, num_sms, stream);
+        if (a.fplan == 2) return fengine_tc_launch(a, tw.tc_image, num_sms, stream);
+        return fengine_launch_rows_a(n_freq, tw, a, num_sms, stream);
     case 18432: case 20480: return fengine_launch_split_a(n_freq, tw, a, num_sms, stream);
     case 22528: case 24576: return fengine_launch_split_b(n_freq, tw, a, num_sms, stream);
     case 26624: case 28672: return fengine_launch_split_c(n_freq, tw, a, num_sms, stream);

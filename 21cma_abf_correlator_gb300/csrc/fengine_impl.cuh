@@ -1,8 +1,8 @@
 // fengine_impl.cuh -- the F-engine's kernel and launch templates, shared by
-// the translation units that instantiate them (fengine.cu and
-// fengine_large.cu / fengine_split_*.cu, one group of transform lengths each,
-// so that they compile in parallel). What the kernel does is described in
-// fengine.cu.
+// the translation units that instantiate them (fengine.cu, fengine_plan1.cu and
+// fengine_split_*.cu, one group of transform lengths each, so that they compile
+// in parallel). What the kernel does is described in fengine.cu. The lengths
+// 4096 .. 16384 have a kernel of their own (fengine_rows.cuh) unless frames are few.
 
 #ifndef CORR_GB300_FENGINE_IMPL_CUH
 #define CORR_GB300_FENGINE_IMPL_CUH
@@ -20,8 +20,14 @@
 namespace corrgb {
 
 // Launchers of the groups of lengths compiled apart from fengine.cu.
-corr_status fengine_launch_large(int n_freq, const TwiddleTables &tw, const FengineArgs &a,
-                                 int num_sms, cudaStream_t stream);   // 10240 .. 16384
+corr_status fengine_launch_rows_a(int n_freq, const TwiddleTables &tw, const FengineArgs &a,
+                                  int num_sms, cudaStream_t stream);  // 14336, 16384
+corr_status fengine_launch_rows_b(int n_freq, const TwiddleTables &tw, const FengineArgs &a,
+                                  int num_sms, cudaStream_t stream);  // 10240, 12288
+corr_status fengine_launch_rows_c(int n_freq, const TwiddleTables &tw, const FengineArgs &a,
+                                  int num_sms, cudaStream_t stream);  // 4096, 6144, 8192
+corr_status fengine_launch_plan1(const TwiddleTables &tw, const FengineArgs &a, int num_sms,
+                                 cudaStream_t stream);                // 16384, FFT plan 1
 corr_status fengine_launch_split_a(int n_freq, const TwiddleTables &tw, const FengineArgs &a,
                                    int num_sms, cudaStream_t stream); // 18432, 20480
 corr_status fengine_launch_split_b(int n_freq, const TwiddleTables &tw, const FengineArgs &a,
@@ -952,10 +958,6 @@ corr_status launch_plan(const FengineArgs &a, const TwiddleTables &tw, int num_s
 template <int MM>
 corr_status launch_size(const FengineArgs &a, const TwiddleTables &tw, int num_sms,
                         cudaStream_t stream) {
-    if constexpr (MM == 16384) {
-        if (a.fplan == 1) return launch_plan<MM, 1>(a, tw, num_sms, stream);
-        if (a.fplan == 2) return fengine_tc_launch(a, tw.tc_image, num_sms, stream);
-    }
     if (a.fplan != 0)
         return failf(CORR_ERR_ARG, "FFT plan %d is not available at n_freq=%d", a.fplan, MM);
     return launch_plan<MM, 0>(a, tw, num_sms, stream);

@@ -106,6 +106,65 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const void *map, int x, i
         : "memory");
 }
 
+// Order tcgen05 operations before / after a thread synchronisation.
+__device__ __forceinline__ void tc_fence_after() {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void tc_fence_before() {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+}
+
+// Tensor memory as per-thread storage: warp w of a CTA reaches lanes
+// [32*(w%4), 32*(w%4)+32), a lane per thread, one 32-bit word per column.
+// alloc/dealloc by one whole warp; n_cols a power of two >= 32. alloc waits while
+// other CTAs on the SM hold too many columns.
+__device__ __forceinline__ void tmem_alloc(uint32_t *smem_base, uint32_t n_cols) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_addr(smem_base)),
+                 "r"(n_cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_dealloc(uint32_t base, uint32_t n_cols) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(n_cols)
+                 : "memory");
+}
+
+// Eight float2 of this thread to / from 16 columns (load: complete only after
+// tmem_wait8, which the values must pass through).
+__device__ __forceinline__ void tmem_store8(uint32_t taddr, const float2 *v) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "f"(v[0].x), "f"(v[0].y), "f"(v[1].x), "f"(v[1].y), "f"(v[2].x), "f"(v[2].y), "f"(v[3].x),
+        "f"(v[3].y), "f"(v[4].x), "f"(v[4].y), "f"(v[5].x), "f"(v[5].y), "f"(v[6].x), "f"(v[6].y),
+        "f"(v[7].x), "f"(v[7].y)
+        : "memory");
+}
+
+__device__ __forceinline__ void tmem_store_wait() {
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_load8(uint32_t taddr, float2 *v) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[2].x), "=f"(v[2].y),
+          "=f"(v[3].x), "=f"(v[3].y), "=f"(v[4].x), "=f"(v[4].y), "=f"(v[5].x), "=f"(v[5].y),
+          "=f"(v[6].x), "=f"(v[6].y), "=f"(v[7].x), "=f"(v[7].y)
+        : "r"(taddr));
+}
+
+__device__ __forceinline__ void tmem_wait8(float2 *v) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0].x), "+f"(v[0].y), "+f"(v[1].x), "+f"(v[1].y), "+f"(v[2].x),
+                   "+f"(v[2].y), "+f"(v[3].x), "+f"(v[3].y), "+f"(v[4].x), "+f"(v[4].y),
+                   "+f"(v[5].x), "+f"(v[5].y), "+f"(v[6].x), "+f"(v[6].y), "+f"(v[7].x),
+                   "+f"(v[7].y));
+}
+
 // *dst += v, performed at L2, with no value returned to the thread.
 __device__ __forceinline__ void red_add_f64(double *dst, double v) {
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(gmem_addr(dst)), "d"(v) : "memory");

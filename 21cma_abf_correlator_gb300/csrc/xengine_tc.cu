@@ -244,14 +244,6 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
         : "memory");
 }
 
-__device__ __forceinline__ void tc_fence_after() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-
 // Issue a 32-lane x 16-column TMEM load without waiting (tmem_ld_wait completes it).
 __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t *r) {
     asm volatile(

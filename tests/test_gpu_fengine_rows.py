@@ -1,0 +1,71 @@
+"""The F-engine of n_freq 4096 .. 16384 (frames in groups of a CTA's warps): few frames
+and ragged counts, frames missing so that the groups get out of step, lost packets.
+
+Tolerance: the plain path's bar against the float64 oracle (1e-5); a misplaced or
+stale point shows at order 1.
+"""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# stations x frames of 1 and 3 leave groups without a frame; 500 and 1201 are a few
+# frames per group on every SM, and one more
+SHAPES = [(1, 1), (3, 1), (1, 500), (1, 1201)]
+
+
+@pytest.mark.parametrize("nf", [4096, 6144, 8192, 10240, 12288, 14336, 16384])
+@pytest.mark.parametrize("n,frames", SHAPES)
+def test_ragged_counts_and_missing_frames(pkg, cuda, oracle, nf, n, frames):
+    torch = cuda
+    rng = np.random.default_rng(nf + frames)
+    x = rng.integers(-128, 128, size=(n, frames, 2 * nf), dtype=np.int16).astype(np.int8)
+    masks = [None]
+    if frames > 1:   # every third frame only; a run missing; all but the last missing
+        f = np.arange(frames)
+        masks += [f % 3 == 0, (f < 100) | (f > 400), f == frames - 1]
+    eng = pkg.FxEngine(n, nf, max_frames=frames, xmode=0)
+    try:
+        xs = torch.from_numpy(x).cuda()
+        for keep in masks:
+            present = None if keep is None else np.broadcast_to(keep, (n, frames))
+            ms = None
+            if present is not None:
+                ms = torch.from_numpy(np.packbits(present.astype(np.uint8), axis=1,
+                                                  bitorder="little")).cuda()
+            acc = eng.new_acc()
+            eng.accumulate(xs, frames, acc, mask=ms)
+            torch.cuda.synchronize()
+            eng.check()
+            ref = oracle.correlate(x, present)
+            assert oracle.rel_rms(acc.cpu().numpy(), ref) < 1e-5
+    finally:
+        eng.close()
+
+
+@pytest.mark.parametrize("nf", [4096, 6144, 10240, 16384])
+def test_every_single_packet(pkg, cuda, oracle, nf):
+    """Frame f keeps only packet f mod the frame's packets."""
+    torch = cuda
+    packets = 2 * nf // 1024
+    frames = packets + 1
+    rng = np.random.default_rng(nf)
+    x = rng.integers(-100, 101, size=(1, frames, 2 * nf)).astype(np.int8)
+    words = np.array([[1 << (f % packets) for f in range(frames)]], dtype=np.uint32)
+    kept = np.zeros_like(x)
+    for f in range(frames):
+        p = f % packets
+        kept[0, f, p * 1024:(p + 1) * 1024] = x[0, f, p * 1024:(p + 1) * 1024]
+    eng = pkg.FxEngine(1, nf, max_frames=frames, xmode=0)
+    try:
+        acc = eng.new_acc()
+        eng.accumulate(torch.from_numpy(x).cuda(), frames, acc,
+                       packets=torch.from_numpy(words.view(np.int32)).cuda())
+        torch.cuda.synchronize()
+        eng.check()
+    finally:
+        eng.close()
+    assert oracle.rel_rms(acc.cpu().numpy(), oracle.correlate(kept)) < 1e-5
