@@ -176,6 +176,13 @@ __device__ __forceinline__ void red_add_f32x2(float2 *dst, float2 v) {
                  : "memory");
 }
 
+// dst[0..3] += {a.x, a.y, b.x, b.y} in FP32, likewise; dst 16-byte aligned.
+__device__ __forceinline__ void red_add_f32x4(float2 *dst, float2 a, float2 b) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(gmem_addr(dst)), "f"(a.x),
+                 "f"(a.y), "f"(b.x), "f"(b.y)
+                 : "memory");
+}
+
 // (double)x in integer arithmetic. This GPU converts (and computes) doubles at
 // 2 lanes per SM and cycle; a normal float only needs its exponent moved.
 __device__ __forceinline__ double widen(float x) {

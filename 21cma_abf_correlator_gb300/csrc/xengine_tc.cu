@@ -48,16 +48,29 @@
 //     (ytile = CT): the stage is one contiguous block and one bulk copy brings
 //     the launch's frames of it; the converters read the rest as zeros.
 //   warps 1..kIssuers (lane 0): the MMAs of a stage once its operands are
-//     written, the operand regions dealt round robin over the issuers.
+//     written, the operand regions dealt round robin over the issuers (as many as
+//     there are regions).
 //   converter warps: regroup a landed stage (FP16 bins, frame-major) into the
 //     K-major no-swizzle operand layout (8-row x 16-byte core matrices, frames
 //     along K) with byte permutes.
 //   last four warps (epilogue, one per TMEM lane quarter): after a tile's last MMA,
 //     read the accumulators (tcgen05.ld), pair rows 2j/2j+1 with one shuffle,
 //     stage V (and Q), release TMEM, then add V into the row in global memory
-//     with 16-byte read-modify-writes (one owner per channel tile and launch).
+//     with reductions at L2 (one owner per channel tile and launch).
 // The roles meet only at mbarriers, all waited on with clock-bounded waits, so
 // a stuck party makes the others time out and report instead of hanging.
+//
+// What bounds it: with 32-byte pieces per (frame, station) row, the spectra's read
+// (5.7 TB/s of a measured 6.8 at 24 inputs, split form); with 16-byte pieces, the
+// tensor-map loads at about one piece per SM and cycle. A stage used to cost every
+// role 1400 cycles whatever its size, most of it integer divisions by the ring
+// depths and stage counts in single-thread loops, now counters. Per 1024 frames on
+// one GB300, complex64 rows, before -> now: 24 inputs, n_freq 16384: FP16 8 x 32
+// tiles 453 -> 347 us (4 x 64: 393 -> 371), split 4 x 32 714 -> 561 us; 20 inputs,
+// n_freq 8192, split 4 x 32 368 -> 251 us; 40 inputs, n_freq 16384, 512 frames, split
+// 2 x 32 1083 -> 811 us. One converter group of seven warps instead of two of three:
+// 357, 564, 262, 834 us. A row update by loads and stores instead of reductions: 8 us
+// more per launch of 32 frames (24 inputs, n_freq 4096: 40 -> 31 us).
 
 #include <algorithm>
 #include <mutex>
@@ -82,12 +95,21 @@ constexpr int kIssuers = 4;
 constexpr int kThreads = 512;
 constexpr int kEpilogue = 128;
 constexpr int kFirstConverterWarp = 1 + kIssuers;
-constexpr int kConverters = kThreads - kEpilogue - 32 * kFirstConverterWarp;
-constexpr int kFirstEpilogueWarp = kFirstConverterWarp + kConverters / 32;
-static_assert(kConverters >= 192 && kFirstEpilogueWarp * 32 + kEpilogue == kThreads, "layout");
+// Two groups of three converter warps take alternate stages: a stage's conversion
+// is a chain of waits, loads, stores and a proxy fence that takes its 1500 cycles
+// however small the stage, so two run at once. (Warp 11 has no part.)
+constexpr int kConvGroups = 2;
+constexpr int kConvWarps = 3;                    // warps per group
+constexpr int kConverters = 32 * kConvWarps;     // threads per group
+constexpr int kFirstEpilogueWarp = 12;
+static_assert(kConvGroups <= 2, "a ring is at least two deep: one step passes its end once");
+static_assert(kFirstConverterWarp + kConvGroups * kConvWarps <= kFirstEpilogueWarp &&
+                  kFirstEpilogueWarp * 32 + kEpilogue == kThreads,
+              "layout");
 constexpr int kMaxLoadStages = 6;
 constexpr int kMaxOpStages = 3;
-constexpr int kMaxItems = 4;                     // conversion items per converter thread
+constexpr int kMaxStageItems = 896;              // conversion items per stage
+constexpr int kMaxItems = (kMaxStageItems + kConverters - 1) / kConverters;   // per thread
 constexpr int kLBO = 128;                        // bytes between K-adjacent core matrices
 // Dynamic shared memory of any feasible shape: the 227 KB a CTA may opt into,
 // less 1 KB left for the kernel's static shared variables.
@@ -191,7 +213,7 @@ TcGeom make_geom(int n_station, bool split, int ct, int kt) {
     g.ld_stage = kt * N * ct * g.elem;
     // paired form: items enumerate stations in groups of four (see the converters)
     g.items = ct * (g.form == kFp16Paired ? round_up(N, 4) : N) * (kt / 8);
-    if (g.items > kMaxItems * kConverters) return g;
+    if (g.items > kMaxStageItems) return g;
     const int n_baseline = N * (N + 1) / 2;
     g.vs_bytes = round_up(n_baseline * ct * 8, 128);
     g.qs_bytes = split ? round_up(N * N * ct * 8, 128) : 0;
@@ -276,14 +298,16 @@ struct TcParams {
     TcGeom g;
 };
 
+// Warps arrive once each (lane 0, after __syncwarp): 32 arrivals of a warp would
+// follow one another.
 struct TcBars {
     uint64_t load_full[kMaxLoadStages];  // a stage's TMA load landed (tx-count)
-    uint64_t load_empty[kMaxLoadStages]; // converters finished reading a slot (256 arrivals)
-    uint64_t op_full[kMaxOpStages];      // converters wrote a stage's operands (256 arrivals)
+    uint64_t load_empty[kMaxLoadStages]; // a converter group finished reading a slot
+    uint64_t op_full[kMaxOpStages];      // a converter group wrote a stage's operands
     uint64_t op_empty[kMaxOpStages];     // MMAs reading an operand buffer finished (commit)
     uint64_t acc_full[2];                // a tile's MMAs finished (commit), per set
-    uint64_t acc_empty[2];               // epilogue read a set (128 arrivals)
-    uint64_t epi;                        // epilogue-only sync (128 arrivals, twice per tile)
+    uint64_t acc_empty[2];               // epilogue read a set
+    uint64_t epi;                        // epilogue-only sync (twice per tile)
     uint64_t fin;                        // abort path: every MMA this CTA issued finished
 };
 
@@ -301,6 +325,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int warp = tid >> 5;
     const int lane = tid & 31;
     const int N = p.n_station;
+    // one issuing thread per operand region, up to kIssuers: each waits for and
+    // commits every stage, so one without MMAs would only lengthen the stage
+    const int n_issuers = min(g.regions, kIssuers);
     const int n_tiles = p.n_freq / g.ct;
     const int my_tiles = (n_tiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) /
                          static_cast<int>(gridDim.x);
@@ -330,18 +357,18 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (tid == 0) {
         for (int s = 0; s < g.n_ld; ++s) {
             mbar_init(&bars.load_full[s], 1);
-            mbar_init(&bars.load_empty[s], kConverters);
+            mbar_init(&bars.load_empty[s], kConvWarps);
         }
         for (int s = 0; s < g.n_op; ++s) {
-            mbar_init(&bars.op_full[s], kConverters);
-            mbar_init(&bars.op_empty[s], kIssuers);
+            mbar_init(&bars.op_full[s], kConvWarps);
+            mbar_init(&bars.op_empty[s], n_issuers);
         }
         for (int s = 0; s < 2; ++s) {
-            mbar_init(&bars.acc_full[s], kIssuers);
-            mbar_init(&bars.acc_empty[s], kEpilogue);
+            mbar_init(&bars.acc_full[s], n_issuers);
+            mbar_init(&bars.acc_empty[s], kEpilogue / 32);
         }
-        mbar_init(&bars.epi, kEpilogue);
-        mbar_init(&bars.fin, kIssuers);
+        mbar_init(&bars.epi, kEpilogue / 32);
+        mbar_init(&bars.fin, n_issuers);
         s_abort = 0;
         s_ld_issued = 0;
         fence_mbar_init();
@@ -368,18 +395,16 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&ymap))
                          : "memory");
+            // slot and phase of the ring, tile and stage: counted, not divided out
+            int slot = 0, st = 0, c0 = tile_c0(0), tile_y = c0 / p.ytile;
+            uint32_t lap = 0;   // times round the ring
             for (int gs = 0; gs < total && *abort_flag == 0; ++gs) {
-                const int tl = gs / n_stages;
-                const int st = gs - tl * n_stages;
-                const int slot = gs % g.n_ld;
-                const int use = gs / g.n_ld;
-                if (use > 0 &&
-                    !mbar_wait_bounded(&bars.load_empty[slot], static_cast<uint32_t>(use - 1) & 1u,
-                                       p.err, kErrXengineMmaTimeout, abort_flag)) {
+                if (lap > 0 &&
+                    !mbar_wait_bounded(&bars.load_empty[slot], (lap - 1) & 1u, p.err,
+                                       kErrXengineMmaTimeout, abort_flag)) {
                     s_abort = 1;
                     break;
                 }
-                const int c0 = tile_c0(tl);
                 if (p.bulk) {
                     // channel tiles of CT bins: the stage's frames x stations x CT
                     // bins are contiguous. Only the launch's frames are copied; the
@@ -396,47 +421,52 @@ __global__ void __launch_bounds__(kThreads, 1)
                     mbar_arrive_expect_tx(&bars.load_full[slot],
                                           static_cast<uint32_t>(g.ld_stage));
                     // frames past `frames` (the map's last frame) arrive as zeros
-                    tma_load_4d(ld_ring + slot * g.ld_stage, &ymap, c0 % p.ytile, 0,
-                                st * g.kt, c0 / p.ytile, &bars.load_full[slot]);
+                    tma_load_4d(ld_ring + slot * g.ld_stage, &ymap, c0 - tile_y * p.ytile, 0,
+                                st * g.kt, tile_y, &bars.load_full[slot]);
                 }
                 ++s_ld_issued;
+                if (++slot == g.n_ld) {
+                    slot = 0;
+                    ++lap;
+                }
+                if (++st == n_stages) {
+                    st = 0;
+                    c0 += static_cast<int>(gridDim.x) * g.ct;
+                    tile_y = c0 / p.ytile;
+                }
             }
         }
     } else if (warp < kFirstConverterWarp) {
         // ------------------------------ MMAs ------------------------------
-        // issuer i: regions i, i + kIssuers, ... Every issuer commits every
-        // stage (op_empty and acc_full count kIssuers arrivals), with or
-        // without MMAs of its own.
+        // issuer i: regions i, i + n_issuers, ... Every issuer commits every stage
+        // (op_empty and acc_full count n_issuers arrivals).
         const int issuer = warp - 1;
-        if (lane == 0) {
+        if (lane == 0 && issuer < n_issuers) {
             const uint32_t idesc = instr_desc_f16_f32(128, g.nb);
             const int ksteps = g.kt / 16;
             // Descriptors differ only in their start-address field, which
             // cannot carry: (address >> 4) of shared memory fits its 14 bits.
             const uint64_t desc0 = smem_desc(smem_addr(op_ring), g.sbo);
+            int ob = 0, st = 0, aset = 0;
+            uint32_t op_lap = 0, acc_lap = 0;   // times round the operand stages, the sets
             for (int gs = 0; gs < total && *abort_flag == 0; ++gs) {
-                const int tl = gs / n_stages;
-                const int st = gs - tl * n_stages;
-                const int ob = gs % g.n_op;
-                const int aset = tl % g.n_acc;
-                const int use = tl / g.n_acc;   // earlier tiles that used this set
-                if (st == 0 && use > 0) {
+                if (st == 0 && acc_lap > 0) {
                     // this set's previous tile must be read before it is overwritten
-                    if (!mbar_wait_bounded(&bars.acc_empty[aset], static_cast<uint32_t>(use - 1) & 1u,
-                                           p.err, kErrXengineMmaTimeout, abort_flag)) {
+                    if (!mbar_wait_bounded(&bars.acc_empty[aset], (acc_lap - 1) & 1u, p.err,
+                                           kErrXengineMmaTimeout, abort_flag)) {
                         s_abort = 1;
                         break;
                     }
                 }
-                if (!mbar_wait_bounded(&bars.op_full[ob], static_cast<uint32_t>(gs / g.n_op) & 1u,
-                                       p.err, kErrXengineMmaTimeout, abort_flag)) {
+                if (!mbar_wait_bounded(&bars.op_full[ob], op_lap & 1u, p.err,
+                                       kErrXengineMmaTimeout, abort_flag)) {
                     s_abort = 1;
                     break;
                 }
                 tc_fence_after();
                 const uint64_t dstage = desc0 + (static_cast<uint32_t>(ob * g.op_stage) >> 4);
                 const uint32_t dset = tmem + static_cast<uint32_t>(aset * g.acc_cols);
-                for (int r = issuer; r < g.regions; r += kIssuers) {
+                for (int r = issuer; r < g.regions; r += n_issuers) {
                     const uint32_t d = dset + static_cast<uint32_t>(r * g.nb);
                     const uint64_t dr =
                         dstage + (static_cast<uint32_t>(r * g.region_stride + region_skew(r)) >> 4);
@@ -446,12 +476,24 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                 }
                 umma_commit(&bars.op_empty[ob]);
-                if (st == n_stages - 1) umma_commit(&bars.acc_full[aset]);
+                if (++ob == g.n_op) {
+                    ob = 0;
+                    ++op_lap;
+                }
+                if (++st == n_stages) {
+                    umma_commit(&bars.acc_full[aset]);
+                    st = 0;
+                    if (++aset == g.n_acc) {
+                        aset = 0;
+                        ++acc_lap;
+                    }
+                }
             }
         }
-    } else if (warp < kFirstEpilogueWarp) {
+    } else if (warp < kFirstConverterWarp + kConvGroups * kConvWarps) {
         // --------------------------- converters ---------------------------
-        const int wt = tid - 32 * kFirstConverterWarp;
+        const int conv_group = (warp - kFirstConverterWarp) / kConvWarps;
+        const int wt = tid - 32 * (kFirstConverterWarp + conv_group * kConvWarps);
         // This thread's items (channel c, station s, 8-frame group kq) are the
         // same every stage: keep their fp32 and operand offsets.
         int n_item = 0;
@@ -504,14 +546,29 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
         const int row_step = N * g.ct;   // float2 between consecutive frames of a slot
-        for (int gs = 0; gs < total; ++gs) {
-            const int lb = gs % g.n_ld;
-            const int ob = gs % g.n_op;
-            bool ok = mbar_wait_bounded(&bars.load_full[lb], static_cast<uint32_t>(gs / g.n_ld) & 1u,
-                                        p.err, kErrXengineMmaTimeout, abort_flag);
-            if (ok && gs >= g.n_op)
-                ok = mbar_wait_bounded(&bars.op_empty[ob],
-                                       static_cast<uint32_t>(gs / g.n_op - 1) & 1u, p.err,
+        // this group's ring slot, operand stage and stage of the tile
+        int lb = conv_group, ob = conv_group, st = conv_group;
+        uint32_t ld_lap = 0, op_lap = 0;
+        auto next_stage = [&] {
+            lb += kConvGroups;
+            if (lb >= g.n_ld) {
+                lb -= g.n_ld;
+                ++ld_lap;
+            }
+            ob += kConvGroups;
+            if (ob >= g.n_op) {
+                ob -= g.n_op;
+                ++op_lap;
+            }
+            st += kConvGroups;
+            while (st >= n_stages) st -= n_stages;
+        };
+        while (st >= n_stages) st -= n_stages;
+        for (int gs = conv_group; gs < total; gs += kConvGroups, next_stage()) {
+            bool ok = mbar_wait_bounded(&bars.load_full[lb], ld_lap & 1u, p.err,
+                                        kErrXengineMmaTimeout, abort_flag);
+            if (ok && op_lap > 0)
+                ok = mbar_wait_bounded(&bars.op_empty[ob], (op_lap - 1) & 1u, p.err,
                                        kErrXengineMmaTimeout, abort_flag);
             if (!ok) {
                 s_abort = 1;
@@ -523,8 +580,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             // Frames of a bulk-loaded last stage past the launch's frames were not
             // copied (stale bytes): they convert as zeros. A tensor-map load
             // zero-fills them itself.
-            const int st_here = gs % n_stages;
-            const int n_valid = p.bulk ? min(g.kt, p.frames - st_here * g.kt) : g.kt;
+            const int n_valid = p.bulk ? min(g.kt, p.frames - st * g.kt) : g.kt;
             auto convert = [&](auto guard_tag) {
                 constexpr bool kGuard = decltype(guard_tag)::value;
                 if (p.in_fmt == kSpectraF16) {
@@ -587,25 +643,29 @@ __global__ void __launch_bounds__(kThreads, 1)
                 convert(std::false_type{});
             else
                 convert(std::true_type{});
-            mbar_arrive(&bars.load_empty[lb]);   // the spectra slot may be refilled
             fence_proxy_async_smem();   // operand stores -> visible to the tensor cores
-            mbar_arrive(&bars.op_full[ob]);
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&bars.load_empty[lb]);   // the spectra slot may be refilled
+                mbar_arrive(&bars.op_full[ob]);
+            }
         }
-    } else {
+    } else if (warp >= kFirstEpilogueWarp) {
         // ---------------------------- epilogue ----------------------------
         const int et = tid - 32 * kFirstEpilogueWarp;
         const int quad = warp & 3;             // TMEM lanes [32*quad, 32*quad+32)
         const int nchunks = (2 * N + 15) / 16;
-        const int nq = g.ct / 2;                // float4 (two channels) per baseline
+        const int nq_shift = __ffs(g.ct) - 2;   // ct/2 float4 (two channels) per baseline
+        const int n_items = n_baseline << nq_shift;
         const int nblk = g.split ? 2 : 1;
         // Staging, one plane per channel, j fastest so that the row lanes of a
         // warp (consecutive j) store to consecutive addresses:
         //   Vt[c][k(k+1)/2 + j] = V[j][k] (j <= k),  Qs[c][k][j] = Q[j][k].
         const int plane_v = n_baseline;
         for (int tl = 0; tl < my_tiles; ++tl) {
-            const int aset = tl % g.n_acc;
-            if (!mbar_wait_bounded(&bars.acc_full[aset], static_cast<uint32_t>(tl / g.n_acc) & 1u,
-                                   p.err, kErrXengineMmaTimeout, abort_flag)) {
+            const int aset = g.n_acc == 2 ? tl & 1 : 0;
+            const int acc_lap = g.n_acc == 2 ? tl >> 1 : tl;
+            if (!mbar_wait_bounded(&bars.acc_full[aset], static_cast<uint32_t>(acc_lap) & 1u, p.err, kErrXengineMmaTimeout, abort_flag)) {
                 s_abort = 1;
                 break;
             }
@@ -668,8 +728,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             // this set is read: the MMAs of tile tl + n_acc may start
             tc_fence_before();
-            mbar_arrive(&bars.acc_empty[aset]);
-            mbar_arrive(&bars.epi);
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&bars.acc_empty[aset]);
+                mbar_arrive(&bars.epi);
+            }
             if (!mbar_wait_bounded(&bars.epi, 0u, p.err, kErrXengineMmaTimeout, abort_flag)) {
                 s_abort = 1;
                 break;
@@ -677,13 +740,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             // V (+ Q[j][k] + conj(Q[k][j])) into the row: this CTA is the only
             // writer of these channels in this launch.
             const int c0 = tile_c0(tl);
-            // Four read-modify-writes per thread in flight: all loads first.
-            constexpr int kBatch = 4;
-            const int n_items = n_baseline * nq;
             // visibilities of channels c, c+1 of item q's baseline
             auto vis = [&](int q, float2 &v0, float2 &v1) {
-                const int b = q / nq;
-                const int c = (q - b * nq) * 2;
+                const int b = q >> nq_shift;
+                const int c = (q - (b << nq_shift)) * 2;
                 const int j = jk[b] >> 8, k = jk[b] & 0xff;
                 const int tri = k * (k + 1) / 2 + j;
                 v0 = Vs[c * plane_v + tri];
@@ -699,50 +759,29 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
             };
             auto row_offset = [&](int q) {
-                const int b = q / nq;
-                const int c = (q - b * nq) * 2;
+                const int b = q >> nq_shift;
+                const int c = (q - (b << nq_shift)) * 2;
                 return static_cast<size_t>(b) * p.n_freq + c0 + c;
             };
-            if (p.acc64) {
-                // complex128 row: the launch's FP32 sums are added in double, as
-                // reductions performed in L2 (red.global.add.f64): this CTA is the
-                // only writer of these values in the launch, so the result is the
-                // same as a read-modify-write, without waiting for the reads.
-                double *acc = static_cast<double *>(p.acc);
-                for (int q = et; q < n_items; q += kEpilogue) {
-                    float2 v0, v1;
-                    vis(q, v0, v1);
-                    double *dst = acc + 2 * row_offset(q);
-                    red_add_f64(dst + 0, v0.x);
-                    red_add_f64(dst + 1, v0.y);
-                    red_add_f64(dst + 2, v1.x);
-                    red_add_f64(dst + 3, v1.y);
-                }
-            } else {
-                float2 *acc = static_cast<float2 *>(p.acc);
-                for (int q0 = et; q0 < n_items; q0 += kEpilogue * kBatch) {
-                    float4 a[kBatch];
-#pragma unroll
-                    for (int u = 0; u < kBatch; ++u) {
-                        const int q = q0 + u * kEpilogue;
-                        if (q < n_items) a[u] = *reinterpret_cast<const float4 *>(acc + row_offset(q));
-                    }
-#pragma unroll
-                    for (int u = 0; u < kBatch; ++u) {
-                        const int q = q0 + u * kEpilogue;
-                        if (q >= n_items) break;
-                        float2 v0, v1;
-                        vis(q, v0, v1);
-                        a[u].x += v0.x;
-                        a[u].y += v0.y;
-                        a[u].z += v1.x;
-                        a[u].w += v1.y;
-                        *reinterpret_cast<float4 *>(acc + row_offset(q)) = a[u];
-                    }
+            // As reductions performed in L2: this CTA is the only writer of these
+            // values in the launch, so the result is that of a read-modify-write,
+            // without waiting for the reads.
+            for (int q = et; q < n_items; q += kEpilogue) {
+                float2 v0, v1;
+                vis(q, v0, v1);
+                if (p.acc64) {   // complex128 row: the launch's FP32 sums are added in double
+                    double *dst = static_cast<double *>(p.acc) + 2 * row_offset(q);
+                    red_add_f64(dst + 0, widen(v0.x));
+                    red_add_f64(dst + 1, widen(v0.y));
+                    red_add_f64(dst + 2, widen(v1.x));
+                    red_add_f64(dst + 3, widen(v1.y));
+                } else {
+                    red_add_f32x4(static_cast<float2 *>(p.acc) + row_offset(q), v0, v1);
                 }
             }
             // everyone done with Vs/Qs before the next tile overwrites them
-            mbar_arrive(&bars.epi);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars.epi);
             if (!mbar_wait_bounded(&bars.epi, 1u, p.err, kErrXengineMmaTimeout, abort_flag)) {
                 s_abort = 1;
                 break;
@@ -752,7 +791,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     tc_fence_before();
     __syncthreads();
-    if (s_abort && warp >= 1 && warp < kFirstConverterWarp && lane == 0) {
+    if (s_abort && warp >= 1 && warp <= n_issuers && lane == 0) {
         // Let every MMA this CTA issued finish before TMEM goes away (bounded;
         // the watchdog code is already recorded). A commit covers the issuing
         // thread's earlier MMAs; fin completes once every issuer committed.
