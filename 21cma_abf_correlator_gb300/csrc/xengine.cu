@@ -375,31 +375,46 @@ __global__ void add64_kernel(double2 *__restrict__ dst, const double2 *__restric
     }
 }
 
-// Two channels per thread: 32 bytes of complex128 in, 16 bytes of complex64 out.
-__global__ void dump64_kernel(float2 *__restrict__ out, size_t out_row,
-                              const double2 *__restrict__ src, size_t src_row,
-                              const int32_t *__restrict__ gmap, const int32_t *__restrict__ lmap,
-                              int n_map, int half_freq, int rows, double s) {
-    const size_t per_row = static_cast<size_t>(n_map) * half_freq;
-    const size_t n = per_row * rows;
-    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += stride) {
-        const int r = static_cast<int>(i / per_row);
-        const size_t q = i - static_cast<size_t>(r) * per_row;
-        const int m = static_cast<int>(q / half_freq);
-        const int c2 = static_cast<int>(q - static_cast<size_t>(m) * half_freq);
-        const int gb = gmap ? gmap[m] : m;
-        const int lb = lmap ? lmap[m] : m;
-        const double2 *a = src + r * src_row + (static_cast<size_t>(lb) * half_freq + c2) * 2;
-        const double2 a0 = a[0], a1 = a[1];
-        float4 v;
-        v.x = static_cast<float>(a0.x * s);
-        v.y = static_cast<float>(a0.y * s);
-        v.z = static_cast<float>(a1.x * s);
-        v.w = static_cast<float>(a1.y * s);
-        *reinterpret_cast<float4 *>(out + r * out_row +
-                                    (static_cast<size_t>(gb) * half_freq + c2) * 2) = v;
+// (float)(v * s), s = s_hi + s_lo. This GPU multiplies and converts doubles at 2
+// lanes per SM and cycle, so v is cut, in integer arithmetic, into its leading 24
+// bits and the next 23 (exact to 2^-46 of v) and multiplied in FP32: the last FMA
+// rounds the product once, as the double one is rounded. Zeros, numbers near or past
+// FP32's range, infinities and NaN go the long way.
+__device__ __forceinline__ float scaled_to_float(double v, float s_hi, float s_lo, double s) {
+    const uint32_t top = static_cast<uint32_t>(__double2hiint(v));
+    const uint32_t low = static_cast<uint32_t>(__double2loint(v));
+    const uint32_t e = (top >> 20) & 0x7ffu;   // 1023 + exponent
+    if (e - 960u > 127u) return static_cast<float>(v * s);   // |v| outside [2^-63, 2^65)
+    const uint32_t sign = top & 0x80000000u;
+    const uint32_t f_exp = (e - 896u) << 23;
+    const float hi = __uint_as_float(sign | f_exp | ((top & 0xfffffu) << 3) | (low >> 29));
+    // the low 29 bits' first 23, in units of hi's last place (the last one also set
+    // if any after it is, so that it decides which way a product rounds)
+    const float frac =
+        __uint_as_float(0x3f800000u | ((low >> 6) & 0x7fffffu) | ((low & 0x3fu) != 0u)) - 1.0f;
+    const float lo = frac * __uint_as_float(sign | (f_exp - (23u << 23)));
+    return fmaf(hi, s_hi, fmaf(hi, s_lo, lo * s_hi));
+}
+
+// Two channels per thread and step: 32 bytes of complex128 in, 16 bytes of complex64
+// out. Bound by those bytes since the arithmetic left the FP64 pipe: 24 inputs, n_freq
+// 16384 48 -> 33 us with its launch, 40 inputs 108 -> 63 us. blockIdx.x = row * n_map + baseline, blockIdx.y strides over its channels.
+__global__ void __launch_bounds__(256)
+    dump64_kernel(float2 *__restrict__ out, size_t out_row, const double2 *__restrict__ src,
+                  size_t src_row, const int32_t *__restrict__ gmap,
+                  const int32_t *__restrict__ lmap, int n_map, int half_freq, float s_hi,
+                  float s_lo, double s) {
+    const int r = blockIdx.x / n_map, m = blockIdx.x - r * n_map;
+    const int gb = gmap ? gmap[m] : m;
+    const int lb = lmap ? lmap[m] : m;
+    const double2 *a = src + r * src_row + static_cast<size_t>(lb) * half_freq * 2;
+    float4 *o = reinterpret_cast<float4 *>(out + r * out_row +
+                                           static_cast<size_t>(gb) * half_freq * 2);
+#pragma unroll 2
+    for (int c = blockIdx.y * 256 + threadIdx.x; c < half_freq; c += gridDim.y * 256) {
+        const double2 a0 = a[2 * c], a1 = a[2 * c + 1];
+        o[c] = make_float4(scaled_to_float(a0.x, s_hi, s_lo, s), scaled_to_float(a0.y, s_hi, s_lo, s),
+                           scaled_to_float(a1.x, s_hi, s_lo, s), scaled_to_float(a1.y, s_hi, s_lo, s));
     }
 }
 
@@ -655,10 +670,17 @@ corr_status dump64_launch(float2 *out, size_t out_row, const double2 *src, size_
                           const int32_t *gmap, const int32_t *lmap, int n_map, int n_freq,
                           int rows, double s, cudaStream_t stream) {
     if (n_freq % 2 != 0) return fail(CORR_ERR_INTERNAL, "dump64: n_freq must be even");
-    const size_t n = static_cast<size_t>(n_map) * (n_freq / 2) * static_cast<size_t>(rows);
-    if (n == 0) return CORR_OK;
-    dump64_kernel<<<grid_for(n, 4096), 256, 0, stream>>>(out, out_row, src, src_row, gmap, lmap,
-                                                          n_map, n_freq / 2, rows, s);
+    const int64_t lines = static_cast<int64_t>(n_map) * rows;
+    if (lines <= 0) return CORR_OK;
+    if (lines > 0x7fffffff) return fail(CORR_ERR_INTERNAL, "dump64: too many rows");
+    // four steps a thread where there are lines enough to fill the GPU
+    const int half = n_freq / 2;
+    const int steps = lines * half >= (1 << 19) ? 4 : 1;
+    const dim3 grid(static_cast<unsigned>(lines),
+                    static_cast<unsigned>((half + 256 * steps - 1) / (256 * steps)));
+    const float s_hi = static_cast<float>(s), s_lo = static_cast<float>(s - s_hi);
+    dump64_kernel<<<grid, 256, 0, stream>>>(out, out_row, src, src_row, gmap, lmap, n_map, half,
+                                            s_hi, s_lo, s);
     return cuda_check(cudaGetLastError(), "dump64_kernel launch");
 }
 
