@@ -22,8 +22,14 @@
 // then runs its 128 steps. Mask bytes (8 frames each) are done by the same
 // threads after the samples.
 //
+// PRNG and COUNTER are bound by integer issue (two or three 64-bit multiplies or
+// shifts, the reduction mod 9 and the packing per sample). With byte dot products for
+// the reduction, the first product as a running sum and four samples packed and offset
+// at once, 24 stations x 512 frames of 32768 samples take 400 us instead of 517 (PRNG)
+// on one GB300. SINE is bound by the FP64 pipe.
+//
 // Integer results are bit-exact with the transmitter. SINE uses IEEE double
-// with every multiply, add and divide rounded separately (no contraction), as
+// with every operation rounded separately (no contraction), as
 // the transmitter's Rust code evaluates it; its sin() is CUDA's, which can
 // differ from the host libm's in the last bit, and that can move the rounded
 // sample only when 4*sin(t) lies within a few ulp of a half-integer.
@@ -49,7 +55,6 @@ struct FrontArgs {
     int station0, n_station, frames, ppf;        // ppf = packets per frame
     int mask_bytes;                              // ceil(frames / 8)
     uint64_t frame0;
-    int pattern;
     uint64_t seed;
     double tone;
     uint64_t start_counter, n_packets;
@@ -61,24 +66,28 @@ struct FrontArgs {
     uint64_t offset[kMaxSt];
 };
 
-// x mod 9 for a 64-bit x without a 64-bit division: 2^24 = 1 (mod 9), so x is
-// congruent to the sum of its three 24-bit digits (< 3 * 2^24).
-__device__ __forceinline__ int mod9(uint64_t x) {
-    const uint32_t r = static_cast<uint32_t>(x & 0xFFFFFFu) +
-                       static_cast<uint32_t>((x >> 24) & 0xFFFFFFu) +
-                       static_cast<uint32_t>(x >> 48);
-    return static_cast<int>(r % 9u);
+// x mod 9, x in two 32-bit words, without a 64-bit division: 2^8 = 4, 2^16 = 7, 2^24 =
+// 1 and 2^32 = 4 (mod 9), so x is congruent to its bytes weighed 1 4 7 1 | 4 7 1 4: two
+// byte dot products, a sum of at most 255 * 29 = 7395. The quotient by 9 of such a sum
+// is (sum * 7282) >> 16 (7282 * 9 = 2^16 + 2; exact up to 2^15).
+__device__ __forceinline__ int mod9(uint32_t lo, uint32_t hi) {
+    const uint32_t r = __dp4a(hi, 0x04010704u, __dp4a(lo, 0x01070401u, 0u));
+    return static_cast<int>(r - 9u * ((r * 7282u) >> 16));
 }
 
-// replay.rs:212-226: the sample at absolute index i.
-__device__ __forceinline__ int prng_sample(int64_t i, uint64_t seed) {
-    uint64_t x = (static_cast<uint64_t>(i) + seed) * 0x9E3779B97F4A7C15ull;
+// replay.rs:212-226: the sample at absolute index i, plus 4, from x = (i + seed) * kPrngStep
+// (consecutive samples: one addition). mod 9 of x >> 8: the bytes of x from the second
+// on, weighed 1 4 7 | 1 4 7 1.
+constexpr uint64_t kPrngStep = 0x9E3779B97F4A7C15ull;
+__device__ __forceinline__ int prng_sample(uint64_t x) {
     x ^= x >> 30;
     x *= 0xBF58476D1CE4E5B9ull;
     x ^= x >> 27;
     x *= 0x94D049BB133111EBull;
     x ^= x >> 31;
-    return mod9(x >> 8) - 4;
+    const uint32_t r = __dp4a(static_cast<uint32_t>(x >> 32), 0x01070401u,
+                              __dp4a(static_cast<uint32_t>(x), 0x07040100u, 0u));
+    return static_cast<int>(r - 9u * ((r * 7282u) >> 16));
 }
 
 __device__ __forceinline__ uint64_t xorshift_step(uint64_t x) {
@@ -147,26 +156,37 @@ __device__ __forceinline__ uint32_t pack4(int b0, int b1, int b2, int b3) {
            ((static_cast<uint32_t>(b2) & 0xFFu) << 16) | ((static_cast<uint32_t>(b3) & 0xFFu) << 24);
 }
 
+// Four values 0 .. 8, less 4 each, as bytes: the top bits keep the borrows apart.
+__device__ __forceinline__ uint32_t pack4_less4(int b0, int b1, int b2, int b3) {
+    const uint32_t lo = static_cast<uint32_t>(b0) + 256u * static_cast<uint32_t>(b1);
+    const uint32_t hi = static_cast<uint32_t>(b2) + 256u * static_cast<uint32_t>(b3);
+    return (((lo + 65536u * hi) | 0x80808080u) - 0x04040404u) ^ 0x80808080u;
+}
+
 // replay.rs:257-264: round(4 sin t) with t = phase + k*tone*2pi/4096, each
 // operation rounded on its own as the host evaluates it.
 __device__ __forceinline__ int sine_sample(double phase, double tone, int k) {
     constexpr double kTau = 6.283185307179586;   // f64 nearest to 2*pi
-    const double step = __ddiv_rn(__dmul_rn(__dmul_rn(static_cast<double>(k), tone), kTau),
-                                  static_cast<double>(kSamplesPerPacket));
+    // the division by 4096 as a product with 2^-12: the same correctly rounded number
+    const double step = __dmul_rn(__dmul_rn(__dmul_rn(static_cast<double>(k), tone), kTau),
+                                  1.0 / kSamplesPerPacket);
     const double t = __dadd_rn(phase, step);
     return static_cast<int>(round(__dmul_rn(sin(t), 4.0)));
 }
 
+// A kernel per pattern: each gets the registers and shared memory it needs.
+template <int PATTERN>
 __global__ void __launch_bounds__(kThreads)
 frontend_kernel(const FrontArgs a) {
-    __shared__ uint64_t jump[32 * kJumpStride];   // T^(128*l), columns, l = 0..31
+    // T^(128*l), columns, l = 0..31
+    __shared__ uint64_t jump[PATTERN == CORRX_PATTERN_COUNTER ? 32 * kJumpStride : 1];
     __shared__ uint64_t scratch[2][64];
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int warps_per_cta = kThreads / 32;
 
-    if (a.pattern == CORRX_PATTERN_COUNTER && a.samples != nullptr) {
+    if (PATTERN == CORRX_PATTERN_COUNTER && a.samples != nullptr) {
         // P = T (one xorshift step), squared 7 times: T^128. Then
         // jump[l] = jump[l-1] * T^128, jump[0] = I.
         const int j = threadIdx.x;
@@ -202,7 +222,7 @@ frontend_kernel(const FrontArgs a) {
             const uint64_t counter = frame * a.ppf + p;
             int8_t *dst = a.samples + si * a.station_stride + f * a.frame_stride +
                           static_cast<size_t>(p) * kSamplesPerPacket;
-            if (a.pattern == CORRX_PATTERN_COUNTER) {
+            if constexpr (PATTERN == CORRX_PATTERN_COUNTER) {
                 // replay.rs:235-249; lane l owns bytes [128 l, 128 l + 128).
                 const uint64_t x0 = counter * 0x9E3779B97F4A7C15ull +
                                     static_cast<uint64_t>(s) * 0x12345678ull;
@@ -217,30 +237,33 @@ frontend_kernel(const FrontArgs a) {
 #pragma unroll
                         for (int t = 0; t < 4; ++t) {
                             x = xorshift_step(x);
-                            b[t] = mod9(x >> 3) - 4;
+                            const uint64_t y = x >> 3;
+                            b[t] = mod9(static_cast<uint32_t>(y), static_cast<uint32_t>(y >> 32));
                         }
-                        w[e] = pack4(b[0], b[1], b[2], b[3]);
+                        w[e] = pack4_less4(b[0], b[1], b[2], b[3]);
                     }
                     store16(out + 16 * q, w[0], w[1], w[2], w[3], a.align);
                 }
-            } else if (a.pattern == CORRX_PATTERN_PRNG) {
+            } else if constexpr (PATTERN == CORRX_PATTERN_PRNG) {
                 // replay.rs:251-256: sample k of the packet is prng_sample(
                 // counter*4096 - delay + k).
                 const int64_t first = static_cast<int64_t>(counter * kSamplesPerPacket) -
                                       frame_delay(a, frame, s);
+                const uint64_t x0 = (static_cast<uint64_t>(first) + a.seed) * kPrngStep;
 #pragma unroll 1
                 for (int q = 0; q < kSamplesPerPacket / 512; ++q) {
                     const int k0 = q * 512 + lane * 16;
                     uint32_t w[4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        w[e] = pack4(prng_sample(first + k0 + 4 * e, a.seed),
-                                     prng_sample(first + k0 + 4 * e + 1, a.seed),
-                                     prng_sample(first + k0 + 4 * e + 2, a.seed),
-                                     prng_sample(first + k0 + 4 * e + 3, a.seed));
+                    for (int e = 0; e < 4; ++e) {
+                        const uint64_t x = x0 + static_cast<uint64_t>(k0 + 4 * e) * kPrngStep;
+                        w[e] = pack4_less4(prng_sample(x), prng_sample(x + kPrngStep),
+                                           prng_sample(x + 2 * kPrngStep),
+                                           prng_sample(x + 3 * kPrngStep));
+                    }
                     store16(dst + k0, w[0], w[1], w[2], w[3], a.align);
                 }
-            } else if (a.pattern == CORRX_PATTERN_SINE) {
+            } else if constexpr (PATTERN == CORRX_PATTERN_SINE) {
                 constexpr double kTau = 6.283185307179586;
                 const double phase = __dmul_rn(
                     __dmul_rn(__dadd_rn(static_cast<double>(counter),
@@ -342,7 +365,6 @@ extern "C" corr_status corrx_frontend_fill(const corrx_frontend *fe, int32_t sta
     a.ppf = static_cast<int>(L / kSamplesPerPacket);
     a.mask_bytes = mask_bytes;
     a.frame0 = static_cast<uint64_t>(frame0);
-    a.pattern = fe->pattern;
     a.seed = fe->seed;
     a.tone = fe->tone;
     a.start_counter = fe->start_counter;
@@ -377,6 +399,10 @@ extern "C" corr_status corrx_frontend_fill(const corrx_frontend *fe, int32_t sta
                                    (bytes + kThreads - 1) / kThreads);
     const uint64_t cap = static_cast<uint64_t>(sms) * 8;
     const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min(want, cap)));
-    frontend_kernel<<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
+    auto kernel = fe->pattern == CORRX_PATTERN_COUNTER ? frontend_kernel<CORRX_PATTERN_COUNTER>
+                  : fe->pattern == CORRX_PATTERN_PRNG  ? frontend_kernel<CORRX_PATTERN_PRNG>
+                  : fe->pattern == CORRX_PATTERN_SINE  ? frontend_kernel<CORRX_PATTERN_SINE>
+                                                       : frontend_kernel<CORRX_PATTERN_ZERO>;
+    kernel<<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
     return cuda_check(cudaGetLastError(), "frontend_kernel launch");
 }
