@@ -557,30 +557,42 @@ corr_status xengine_plain_launch(const XengineArgs &a, int num_sms, cudaStream_t
     const int n_ct = a.n_freq / kXch;
     p.n_parts = plain_parts(a.n_freq, a.frames);
     p.seg = ((a.frames + p.n_parts - 1) / p.n_parts + 1) / 2 * 2;
+    // Ring: four slots (eight if they are small), each as long as fits; rows past
+    // the last station are read (and dropped) by the last tile, hence the pad.
+    const size_t pad = static_cast<size_t>(kTile) * kXch * sizeof(float2);
+    const size_t run_pair = static_cast<size_t>(2) * N * kXch * sizeof(float2);
+    auto budget_of = [&](int slots_p, int slots_c, int ctas) -> size_t {
+        const size_t sums =
+            p.n_parts > 1 ? static_cast<size_t>(p.tiles) * slots_c * kSumElems * sizeof(float2) : 0;
+        const size_t sm = static_cast<size_t>(224 * 1024) / ctas, fixed = 2048 + pad + sums;
+        return sm > fixed && (run_pair * slots_p * slots_c << 2) <= sm - fixed ? sm - fixed : 0;
+    };
     // CTA shape: every tile of a channel tile if they fit, in tile groups (that
     // read the same spectra) otherwise; then parts side by side; then channel
-    // tiles, as long as each SM still gets a CTA.
+    // tiles, as long as each SM still gets a CTA. Not wider than the ring has room
+    // for (a few baselines of many stations: few tiles, long runs).
     p.tile_groups = (p.n_tiles + kMaxWarps - 1) / kMaxWarps;
     p.tiles = (p.n_tiles + p.tile_groups - 1) / p.tile_groups;
     p.slots_p = 1;
-    while (p.slots_p < p.n_parts && p.tiles * p.slots_p * 2 <= kMaxWarps) p.slots_p *= 2;
+    while (p.slots_p < p.n_parts && p.tiles * p.slots_p * 2 <= kMaxWarps &&
+           budget_of(p.slots_p * 2, 1, 1) > 0)
+        p.slots_p *= 2;
     p.slots_c = 1;
     while (p.tiles * p.slots_p * (p.slots_c + 1) <= kMaxWarps &&
-           (n_ct + p.slots_c) / (p.slots_c + 1) * p.tile_groups >= num_sms)
+           (n_ct + p.slots_c) / (p.slots_c + 1) * p.tile_groups >= num_sms &&
+           budget_of(p.slots_p, p.slots_c + 1, 1) > 0)
         ++p.slots_c;
     p.units = (n_ct + p.slots_c - 1) / p.slots_c * p.tile_groups;
     place_tiles(tiles, &p);
-    // Ring: four slots (eight if they are small), each as long as fits; rows past
-    // the last station are read (and dropped) by the last tile, hence the pad.
-    const size_t per_pair = static_cast<size_t>(2) * N * kXch * sizeof(float2) * p.slots_p * p.slots_c;
-    const size_t pad = static_cast<size_t>(kTile) * kXch * sizeof(float2);
+    const size_t per_pair = run_pair * p.slots_p * p.slots_c;
     const int warps = p.tiles * p.slots_p * p.slots_c + 1;
-    const int per_sm = std::max(1, (kMaxWarps + 1) / warps);
-    const size_t sums = p.n_parts > 1 ? p.tiles * p.slots_c * kSumElems * sizeof(float2) : 0;
-    const size_t budget = static_cast<size_t>(224 * 1024) / per_sm - 2048 - pad - sums;
-    p.slot_shift = 8 * 16 * per_pair <= budget ? 3 : 2;
-    if ((per_pair << p.slot_shift) > budget)
+    int per_sm = std::max(1, (kMaxWarps + 1) / warps);
+    while (per_sm > 1 && budget_of(p.slots_p, p.slots_c, per_sm) == 0) --per_sm;
+    const size_t budget = budget_of(p.slots_p, p.slots_c, per_sm);
+    if (budget == 0)
         return failf(CORR_ERR_ARG, "plain X-engine: %d stations do not fit in shared memory", N);
+    const size_t sums = p.n_parts > 1 ? p.tiles * p.slots_c * kSumElems * sizeof(float2) : 0;
+    p.slot_shift = 8 * 16 * per_pair <= budget ? 3 : 2;
     p.fs = 2 * static_cast<int>(std::min<size_t>(16, (budget >> p.slot_shift) / per_pair));
     const size_t ring = ((per_pair * (p.fs / 2)) << p.slot_shift) + pad;
     p.sums_at = static_cast<int>(ring / sizeof(float2));

@@ -12,6 +12,8 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
+from abi_driver import drive_rows
+
 pytestmark = pytest.mark.gpu
 
 CASES = [(1, 512, 1), (3, 512, 2), (4, 1024, 33), (6, 512, 300), (7, 2048, 17), (9, 1024, 64),
@@ -63,3 +65,19 @@ def test_rows_do_not_depend_on_timing(pkg, cuda):
         eng.check()
         eng.close()
         assert all(torch.equal(rows[0], r) for r in rows[1:])
+
+
+def test_few_tiles_of_long_rows(pkg, cuda, oracle):
+    """18 stations, n_freq 32768 over eight devices by baseline range: the last one
+    computes one tile, which as many channel tiles side by side as there are warps
+    would not fit in shared memory. The rows are one device's, bit for bit."""
+    n, nf, frames = 18, 32768, 8
+    x = np.random.default_rng(18).integers(-60, 61, size=(1, n, frames, 2 * nf)).astype(np.int8)
+    one = drive_rows(pkg, x, frames, frames)
+    pkg.set_device_map([0] * 8)
+    try:
+        split = drive_rows(pkg, x, frames, frames, devices=list(range(8)), split_mode=0)
+    finally:
+        pkg.set_device_map(None)
+    assert oracle.normalized_max_err(one[0], oracle.correlate(x[0]), n) < 1e-5
+    assert split.tobytes() == one.tobytes()
