@@ -87,8 +87,8 @@ struct FrCfg {
     static constexpr int OFF_D = OFF_T + ROWS * TROW;
     static constexpr int GROUP = OFF_D + ROWS * DROW * 8;
     static constexpr int OFF_BAR = G * GROUP;      // three mbarriers per group
-    static constexpr int OFF_FLAG = OFF_BAR + 3 * 8 * G;
-    static constexpr int SMEM = OFF_FLAG + 8;
+    static constexpr int OFF_FLAG = OFF_BAR + 3 * 8 * G;   // two words per group
+    static constexpr int SMEM = OFF_FLAG + 8 * G;
     static_assert(SMEM <= 227 * 1024 && GROUP % 16 == 0, "shared memory");
     // the twiddle tables the tensor-memory ones are made from, before the first frame
     static_assert((128 + 2 * (M / 64)) * 8 <= GROUP, "tables fit in a group's memory");
@@ -230,7 +230,9 @@ __global__ void __launch_bounds__(512, 1) fengine_rows_kernel(FengineArgs a, TwP
     float2 *const sd = reinterpret_cast<float2 *>(raw + C::OFF_D);
     uint64_t *const bar = reinterpret_cast<uint64_t *>(smem + C::OFF_BAR) + 3 * g;
     uint64_t *const data_read = bar + 1, *const samples_read = bar + 2;
-    volatile int *const abort_flag = reinterpret_cast<volatile int *>(smem + C::OFF_FLAG);
+    // A wait of frame n that ran out sets word n & 1 of its group before the threads
+    // meet, and all of them look at it after: they leave together, none at a barrier.
+    volatile int *const abort_flag = reinterpret_cast<volatile int *>(smem + C::OFF_FLAG) + 2 * g;
     __shared__ uint32_t s_tmem;
     __shared__ volatile uint32_t entered[4];   // frames each group has taken into the last pass
     const float out_scale = (FMT == kSpectraF32) ? 1.0f : a.y_scale;   // FP32 bins unscaled
@@ -249,7 +251,7 @@ __global__ void __launch_bounds__(512, 1) fengine_rows_kernel(FengineArgs a, TwP
         mbar_init(bar, 1);
         mbar_init(data_read, C::WPF);
         mbar_init(samples_read, C::WPF);
-        *abort_flag = 0;
+        abort_flag[0] = abort_flag[1] = 0;
         entered[g] = 0;
         fence_mbar_init();
     }
@@ -298,8 +300,8 @@ __global__ void __launch_bounds__(512, 1) fengine_rows_kernel(FengineArgs a, TwP
     uint32_t parity = 0;
     const uint32_t raw_at = smem_addr(raw), t_at = raw_at + C::OFF_T;
     // The landed frame to rows. Points of lost packets (512 points, 32 a) become zeros.
-    auto deinterleave = [&](int item) {
-        if (!mbar_wait_bounded(bar, parity, a.err, kErrFengineCopyTimeout)) *abort_flag = 1;
+    auto deinterleave = [&](int item, uint32_t n) {
+        if (!mbar_wait_bounded(bar, parity, a.err, kErrFengineCopyTimeout)) abort_flag[n & 1] = 1;
         parity ^= 1u;
         const int f = item / a.n_station;
         const uint32_t kept = packets_kept<M>(a, f, item - f * a.n_station);
@@ -329,7 +331,7 @@ __global__ void __launch_bounds__(512, 1) fengine_rows_kernel(FengineArgs a, TwP
     issue(cur);
     int nxt = n_items;
     if (cur < n_items) {
-        deinterleave(cur);
+        deinterleave(cur, 0);
         nxt = next_present(cur + stride);
         meet();
         issue(nxt);
@@ -373,7 +375,7 @@ __global__ void __launch_bounds__(512, 1) fengine_rows_kernel(FengineArgs a, TwP
             for (int w = 0; w < RPW; ++w) dft_from_int8<R0>(v[w]);
             // the data of the frame before must be read
             if (n > 0 && !mbar_wait_bounded(data_read, (n - 1) & 1, a.err, kErrFengineCopyTimeout))
-                *abort_flag = 1;
+                abort_flag[n & 1] = 1;
             __syncwarp();
             // k1-major, lane (not a0) fastest: both sides free of bank conflicts
 #pragma unroll
@@ -388,8 +390,8 @@ __global__ void __launch_bounds__(512, 1) fengine_rows_kernel(FengineArgs a, TwP
             for (int r = 0; r < 32; ++r) v[r] = lrow[k1 * 33 + 4 * (r & 7) + (r >> 3)];   // a0 = r
             if (nxt < n_items) {
                 if (!mbar_wait_bounded(samples_read, n & 1, a.err, kErrFengineCopyTimeout))
-                    *abort_flag = 1;
-                deinterleave(nxt);
+                    abort_flag[n & 1] = 1;
+                deinterleave(nxt, n);
             }
             tmem_twiddles<32>(v, tm_lane);
             Dft<32>::run(v);
@@ -400,7 +402,7 @@ __global__ void __launch_bounds__(512, 1) fengine_rows_kernel(FengineArgs a, TwP
             }
         }
         meet();
-        if (*abort_flag) {   // let the copy in flight, if any, land
+        if (abort_flag[n & 1]) {   // let the copy in flight, if any, land
             if (t == 0 && nxt < n_items) mbar_wait_bounded(bar, parity ^ 1u, nullptr, 0);
             break;
         }
