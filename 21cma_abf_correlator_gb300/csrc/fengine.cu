@@ -12,11 +12,9 @@
 //     as zeros, which is what zeroing the samples and transforming them gives;
 //   * the real frame x[0..L) (L = 2M) is packed as M complex points
 //     z[n] = x[2n] + i*x[2n+1] and transformed by a Stockham autosort FFT in
-//     shared memory (three or four passes of radix 4..32, led by an odd radix
-//     3..15 when M is not a power of two; FePlan in fengine_impl.cuh), FP32 in
-//     registers, twiddles from host-computed double-precision tables; above
-//     n_freq 16384 the M points are first split into two M/2-point sequences
-//     (even and odd bins) that the CTA transforms in turn (HALF);
+//     shared memory (three or four passes of radix 4..32, led by radix 3
+//     at 6144; FePlan in fengine_impl.cuh), FP32 in registers, twiddles from
+//     host-computed double-precision tables;
 //   * the split X[k] = Fe[k] + w^k Fo[k] turns Z into the L-point real spectrum;
 //     bins 0..M-1 are written, the Nyquist bin M is dropped and nothing is
 //     normalised (reference semantics, HANDOFF.md:583-602).
@@ -33,7 +31,7 @@
 
 // This file: the host side (twiddle tables, plans, dispatch by length) and the
 // kernels of n_freq 512 .. 2048 and, for few frames, of 4096 .. 8192; fengine_impl.cuh
-// holds the kernel templates, fengine_rows.cuh those of 4096 .. 16384.
+// holds the kernel templates, fengine_rows.cuh those of 4096 .. 16384, fengine_rows_half.cuh those above.
 
 namespace corrgb {
 

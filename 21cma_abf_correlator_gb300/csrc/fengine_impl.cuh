@@ -409,34 +409,18 @@ __device__ __forceinline__ void apply_twiddles(float2 *v, int u, const float2 *l
 // (R0 x R1 x R2, R1b = 1); plan 1, where a size has one, has four
 // (R0 x R1 x R1b x R2) with half the points per thread and twice the threads:
 // one more shared-memory pass against twice the warps to hide latency. The
-// autotuner times both. A length of 3, 5 or 7 x 2^k (the multiples of 2048 up
-// to 16384 that are not powers of two: a frame of whole 4096-sample packets)
-// starts with that odd radix, whose pass has no twiddles, then three
-// power-of-two passes.
+// autotuner times both. 6144 = 3 x 2^11 starts with the odd radix, whose pass has
+// no twiddles, then three power-of-two passes.
 template <int M, int PLAN>
 struct FePlan;
-template <> struct FePlan<16384, 0> { static constexpr int R0 = 32, R1 = 32, R1b = 1, R2 = 16; };
 template <> struct FePlan<16384, 1> { static constexpr int R0 = 16, R1 = 16, R1b = 8, R2 = 8; };
-template <> struct FePlan<14336, 0> { static constexpr int R0 = 7, R1 = 16, R1b = 8, R2 = 16; };
-template <> struct FePlan<12288, 0> { static constexpr int R0 = 3, R1 = 32, R1b = 8, R2 = 16; };
-template <> struct FePlan<10240, 0> { static constexpr int R0 = 5, R1 = 16, R1b = 8, R2 = 16; };
 template <> struct FePlan<8192, 0> { static constexpr int R0 = 32, R1 = 16, R1b = 1, R2 = 16; };
 template <> struct FePlan<6144, 0> { static constexpr int R0 = 3, R1 = 16, R1b = 8, R2 = 16; };
 template <> struct FePlan<4096, 0> { static constexpr int R0 = 16, R1 = 16, R1b = 1, R2 = 16; };
 template <> struct FePlan<2048, 0> { static constexpr int R0 = 16, R1 = 8, R1b = 1, R2 = 16; };
 template <> struct FePlan<1024, 0> { static constexpr int R0 = 16, R1 = 8, R1b = 1, R2 = 8; };
 template <> struct FePlan<512, 0> { static constexpr int R0 = 16, R1 = 4, R1b = 1, R2 = 8; };
-// Half lengths of n_freq 18432, 22528, 26624 and 30720 (the other half lengths
-// above, 10240 .. 16384, use their own plans).
-template <> struct FePlan<15360, 0> { static constexpr int R0 = 15, R1 = 16, R1b = 4, R2 = 16; };
-template <> struct FePlan<13312, 0> { static constexpr int R0 = 13, R1 = 16, R1b = 4, R2 = 16; };
-template <> struct FePlan<11264, 0> { static constexpr int R0 = 11, R1 = 16, R1b = 4, R2 = 16; };
-template <> struct FePlan<9216, 0> { static constexpr int R0 = 9, R1 = 16, R1b = 4, R2 = 16; };
-
-// HALF: MM is half of n_freq; a CTA holds the whole frame of 4*MM int8 samples
-// (one buffer: two would not fit beside the data) and transforms its two
-// half-length sequences one after the other.
-template <int MM, int PLAN, bool HALF = false>
+template <int MM, int PLAN>
 struct FeCfg {
     using Plan = FePlan<MM, PLAN>;
     static constexpr int M = MM;
@@ -449,11 +433,11 @@ struct FeCfg {
     static constexpr int PADSHIFT = (R0 == 32) ? 5 : 4;
     static constexpr int N_PASS_HI = M / 64;
     static constexpr int N_POST_HI = M / 64;
-    static constexpr int FRAME = HALF ? 4 * M : 2 * M;   // int8 bytes of one frame
+    static constexpr int FRAME = 2 * M;   // int8 bytes of one frame
     // shared memory layout (bytes)
     static constexpr int OFF_X0 = 0;                      // int8 frame, buffer 0
-    static constexpr int OFF_X1 = HALF ? 0 : FRAME;       // int8 frame, buffer 1
-    static constexpr int OFF_D = HALF ? FRAME : 2 * FRAME;   // padded complex data
+    static constexpr int OFF_X1 = FRAME;       // int8 frame, buffer 1
+    static constexpr int OFF_D = 2 * FRAME;   // padded complex data
     static constexpr int OFF_PLO = OFF_D + (M + (M >> PADSHIFT)) * 8;
     static constexpr int OFF_PHI = OFF_PLO + 92 * 8;   // lo[64] + lo4[16] + lo8[8] + lo16[4]
     static constexpr int OFF_QLO = OFF_PHI + N_PASS_HI * 8;
@@ -461,7 +445,6 @@ struct FeCfg {
     static constexpr int OFF_T2 = OFF_QHI + N_POST_HI * 8;   // second-pass twiddles
     static constexpr int OFF_BAR = (OFF_T2 + R0 * R1 * 8 + 15) / 16 * 16;
     static constexpr int OFF_FLAG = OFF_BAR + 16;
-    static constexpr int OFF_SHIFT = OFF_FLAG + 8;        // HALF: odd_shift
     static constexpr int SMEM = OFF_FLAG + 16;
     static_assert(SMEM <= 227 * 1024, "shared memory");
     // CTAs per SM the launch bounds plan for: as many as shared memory allows,
@@ -506,37 +489,24 @@ __device__ __forceinline__ int mod_c(int j) {
 }
 
 // Where a pass reads its input: the data in shared memory, or (first pass)
-// the int8 frame: its M sample pairs as M complex points; or, for a frame of
-// 2M pairs split into two half-length sequences (one radix-2 step of
-// decimation in frequency, z = the 2M points), z[e] + z[e+M] (the sequence
-// whose transform is the even bins) or (z[e] - z[e+M]) * exp(-pi*i*e/M) (the
-// odd bins).
-enum PassSource : int { kFromShared = 0, kFromInt8 = 1, kFromInt8Sum = 2, kFromInt8Diff = 3 };
+// the int8 frame: its M sample pairs as M complex points.
+enum PassSource : int { kFromShared = 0, kFromInt8 = 1 };
 
 // Stockham pass of radix R over M points with sub-transform size NS:
 //   out[(j/NS)*NS*R + j%NS + r*NS] = DFT_R( in[j + r*M/R] * w^(r*(j%NS)) )
 // for the M/R butterflies j. Each thread owns ceil(P/R) of them (j = tid + q*T);
 // where R does not divide P (an odd first radix) the last round of butterflies
 // is partial and the threads past M/R sit it out. In place: read all, barrier,
-// write all, barrier. The odd-radix first pass of a split frame (which also
-// combines two points and, for the odd bins, multiplies each by a twiddle)
-// reads the int8 frame, not the data it writes, so it instead waits once at
-// the start (for the previous transform's last reads of the data) and then
-// writes each butterfly as soon as it is computed, holding R values at a time
-// instead of ceil(P/R)*R. (The plain odd-radix first pass keeps the first
-// order: streaming it made n_freq 6144 5 % slower and 10240, 14336 no faster.)
+// write all, barrier.
 // TAB: the pass's twiddles w^(r*(j%NS)) (NS*R of them) come from table `t2`
-// laid out [r][j%NS] instead of from the two-level tables. qlo/qhi: the
-// exp(-pi*i*e/M) tables that kFromInt8Diff multiplies by.
+// laid out [r][j%NS] instead of from the two-level tables.
 template <int M, int T, int P, int R, int NS, int SHIFT, int SRC, bool TAB = false>
 __device__ __forceinline__ void fft_pass(float2 *__restrict__ sd, const char2 *__restrict__ sx,
                                          const float2 *lo, const float2 *hi, int tid,
-                                         const float2 *t2 = nullptr, const float2 *qlo = nullptr,
-                                         const float2 *qhi = nullptr) {
+                                         const float2 *t2 = nullptr) {
     constexpr int NB = (P + R - 1) / R;
     constexpr int STRIDE = M / R;
     constexpr bool EXACT = NB * R == P;   // NB*T == M/R: every thread has NB butterflies
-    constexpr bool STREAM = (SRC == kFromInt8Sum || SRC == kFromInt8Diff) && (R % 2 == 1);
     static_assert(M % (NS * R) == 0, "bad radix plan");
     // Reads: a padded per-thread base plus a compile-time offset, since the read
     // stride is a multiple of the padding period. Writes likewise when the write
@@ -560,21 +530,6 @@ __device__ __forceinline__ void fft_pass(float2 *__restrict__ sd, const char2 *_
         } else if constexpr (SRC == kFromInt8) {
 #pragma unroll
             for (int r = 0; r < R; ++r) v[r] = int8_pair_to_float2(x16[j + r * STRIDE]);
-        } else if constexpr (SRC == kFromInt8Sum) {
-            // with the offset B still in: x[e] + (x[e+M] - 2B) and x[e] - x[e+M]
-            // are the integer sum and difference, exactly (Dft<4>::run_biased)
-            const float2 two_b = make_float2(2.0f * kInt8Bias, 2.0f * kInt8Bias);
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                v[r] = cadd(int8_pair_to_biased(x16[j + r * STRIDE]),
-                            csub(int8_pair_to_biased(x16[j + r * STRIDE + M]), two_b));
-        } else if constexpr (SRC == kFromInt8Diff) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const int e = j + r * STRIDE;
-                v[r] = cmul(csub(int8_pair_to_biased(x16[e]), int8_pair_to_biased(x16[e + M])),
-                            cmul(qlo[e & 63], qhi[e >> 6]));
-            }
         } else {
             const int pj = padi<SHIFT>(j);
 #pragma unroll
@@ -605,33 +560,20 @@ __device__ __forceinline__ void fft_pass(float2 *__restrict__ sd, const char2 *_
             for (int r = 0; r < R; ++r) sd[padi<SHIFT>(base + r * NS)] = v[r];
         }
     };
-    if constexpr (STREAM) {
-        __syncthreads();
+    float2 v[NB][R];
 #pragma unroll
-        for (int q = 0; q < NB; ++q) {
-            const int j = tid + q * T;
-            if (!EXACT && j >= STRIDE) continue;
-            float2 v[R];
-            gather(j, v);
-            transform(v);
-            store(j, v);
-        }
-    } else {
-        float2 v[NB][R];
+    for (int q = 0; q < NB; ++q) {
+        const int j = tid + q * T;
+        if (!EXACT && j >= STRIDE) continue;
+        gather(j, v[q]);
+        transform(v[q]);
+    }
+    __syncthreads();
 #pragma unroll
-        for (int q = 0; q < NB; ++q) {
-            const int j = tid + q * T;
-            if (!EXACT && j >= STRIDE) continue;
-            gather(j, v[q]);
-            transform(v[q]);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < NB; ++q) {
-            const int j = tid + q * T;
-            if (!EXACT && j >= STRIDE) continue;
-            store(j, v[q]);
-        }
+    for (int q = 0; q < NB; ++q) {
+        const int j = tid + q * T;
+        if (!EXACT && j >= STRIDE) continue;
+        store(j, v[q]);
     }
     __syncthreads();
 }
@@ -693,54 +635,15 @@ __device__ __forceinline__ void last_pass_store(const float2 *__restrict__ sd,
     if (t0) yrow.put(M / 2, make_float2(a[H].x * yrow.scale, -a[H].y * yrow.scale));
 }
 
-// Last pass for the odd bins of a frame split into two half-length sequences:
-// B[k'] = Z[2k'+1], k' < M (M = n_freq/2, this transform's length). Bin
-// k = 2k'+1 of the real spectrum pairs with n_freq - k = 2(M-1-k')+1, that is
-// B[k'] with B[M-1-k']; for k' = j + i*J the partner is butterfly J-1-j, output
-// R-1-i. Thread t owns butterflies t and J-1-t (t < J/2 = T), so its R pairs
-// are (a[i], b[R-1-i]) and no element pairs with itself. The split twiddle is
-// exp(-2*pi*i*k/(2*n_freq)) = exp(-pi*i*k'/M) * exp(-pi*i/n_freq) (odd_shift).
-// Row: a STEP 2 row of the odd bins, so index k' lands on bin 2k'+1.
-template <int MM, int PLAN, class Row>
-__device__ __forceinline__ void last_pass_store_odd(const float2 *__restrict__ sd,
-                                                    const float2 *plo, const float2 *phi,
-                                                    const float2 *qlo, const float2 *qhi,
-                                                    float2 odd_shift, const Row &yrow, int tid) {
-    using C = FeCfg<MM, PLAN>;
-    constexpr int M = C::M, J = C::J, R = C::R2;
-    static_assert(J % (1 << C::PADSHIFT) == 0 && J % 2 == 0, "last-pass stride");
-    constexpr int PJ = J + (J >> C::PADSHIFT);
-    const int j1 = tid, j2 = J - 1 - tid;
-    float2 a[R], b[R];
-    const int p1 = padi<C::PADSHIFT>(j1), p2 = padi<C::PADSHIFT>(j2);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        a[r] = sd[p1 + r * PJ];
-        b[r] = sd[p2 + r * PJ];
-    }
-    apply_twiddles<R>(a, j1, plo, phi);
-    apply_twiddles<R>(b, j2, plo, phi);
-    Dft<R>::run(a);   // a[r] = B[j1 + r*J]
-    Dft<R>::run(b);   // b[r] = B[j2 + r*J]
-    const float2 w1 = scale_tw(cmul(cmul(qlo[j1 & 63], qhi[j1 >> 6]), odd_shift), yrow.half);
-#pragma unroll
-    for (int i = 0; i < R; ++i)   // exp(-pi*i*i/R) = exp(-2*pi*i*i*(16/R)/32)
-        split_store(a[i], b[R - 1 - i], mul_w32(w1, i * (16 / R)), j1 + i * J, M - 1, true, yrow);
-}
-
 struct TwPtrs {
     const float2 *pass_lo, *pass_hi, *post_lo, *post_hi;
-    const float2 *odd_shift;   // HALF only
+    const float2 *odd_shift;   // n_freq above 16384 only
 };
 
-// HALF (n_freq = 2*MM above 16384): each item's frame of 2*MM sample pairs is
-// transformed as two MM-point sequences, even bins then odd bins, from one
-// int8 buffer; the next item's copy is issued once the second sequence's first
-// pass has read the frame, and lands during the rest of that transform.
-template <int MM, int PLAN, int FMT, bool CONTIG, bool HALF>
-__global__ void __launch_bounds__(FeCfg<MM, PLAN, HALF>::T, FeCfg<MM, PLAN, HALF>::MIN_BLOCKS)
+template <int MM, int PLAN, int FMT, bool CONTIG>
+__global__ void __launch_bounds__(FeCfg<MM, PLAN>::T, FeCfg<MM, PLAN>::MIN_BLOCKS)
     fengine_kernel(FengineArgs a, TwPtrs tw) {
-    using C = FeCfg<MM, PLAN, HALF>;
+    using C = FeCfg<MM, PLAN>;
     constexpr int M = C::M;
     constexpr int T = C::T;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -754,10 +657,8 @@ __global__ void __launch_bounds__(FeCfg<MM, PLAN, HALF>::T, FeCfg<MM, PLAN, HALF
     float2 *t2 = reinterpret_cast<float2 *>(smem + C::OFF_T2);
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + C::OFF_BAR);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + C::OFF_FLAG);
-    float2 *odd_shift = reinterpret_cast<float2 *>(smem + C::OFF_SHIFT);
 
     const int tid = threadIdx.x;
-    if (HALF && tid == 0) *odd_shift = *tw.odd_shift;
     for (int i = tid; i < 64; i += T) {
         plo[i] = tw.pass_lo[i];
         qlo[i] = tw.post_lo[i];
@@ -776,7 +677,7 @@ __global__ void __launch_bounds__(FeCfg<MM, PLAN, HALF>::T, FeCfg<MM, PLAN, HALF
     }
     if (tid == 0) {
         mbar_init(&bar[0], 1);
-        if (!HALF) mbar_init(&bar[1], 1);
+        mbar_init(&bar[1], 1);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -805,10 +706,10 @@ __global__ void __launch_bounds__(FeCfg<MM, PLAN, HALF>::T, FeCfg<MM, PLAN, HALF
     uint32_t parity_bits = 0u;   // bit b = phase parity of bar[b]
 
     for (int n = 0; item < n_items; ++n, item += gridDim.x) {
-        const int buf = HALF ? 0 : (n & 1);
+        const int buf = n & 1;
         const int next = item + gridDim.x;
         bool next_issued = false;
-        if (!HALF && tid == 0 && next < n_items && present(next)) {
+        if (tid == 0 && next < n_items && present(next)) {
             // The other buffer was last read by the previous item's first pass,
             // which every thread finished before that pass's first barrier.
             fence_proxy_async_smem();
@@ -816,15 +717,6 @@ __global__ void __launch_bounds__(FeCfg<MM, PLAN, HALF>::T, FeCfg<MM, PLAN, HALF
             bulk_copy_g2s(buf ? sx0 : sx1, src_of(next), frame_bytes, &bar[buf ^ 1]);
             next_issued = true;
         }
-        // HALF: the single buffer is free once this item's frame has been read
-        // (or at once, for a missing frame, which was never copied).
-        auto issue_next_into_buffer = [&] {
-            if (tid == 0 && next < n_items && present(next)) {
-                fence_proxy_async_smem();
-                mbar_arrive_expect_tx(&bar[0], frame_bytes);
-                bulk_copy_g2s(sx0, src_of(next), frame_bytes, &bar[0]);
-            }
-        };
         using Row = YRow<FMT, CONTIG>;
         const Row yrow{
             reinterpret_cast<typename Row::T *>(a.y) + static_cast<size_t>(item) * a.ytile,
@@ -832,9 +724,8 @@ __global__ void __launch_bounds__(FeCfg<MM, PLAN, HALF>::T, FeCfg<MM, PLAN, HALF
             0.5f * out_scale};
 
         if (!present(item)) {
-            if constexpr (HALF) issue_next_into_buffer();
             // Missing frame: its samples count as zeros, so does its spectrum.
-            for (int k = tid; k < (HALF ? 2 * M : M); k += T) yrow.put(k, make_float2(0.f, 0.f));
+            for (int k = tid; k < M; k += T) yrow.put(k, make_float2(0.f, 0.f));
             continue;
         }
 
@@ -846,32 +737,6 @@ __global__ void __launch_bounds__(FeCfg<MM, PLAN, HALF>::T, FeCfg<MM, PLAN, HALF
                                kErrFengineCopyTimeout))
             *abort_flag = 1;
         parity_bits ^= 1u << buf;
-
-        if constexpr (HALF) {
-            using RowH = YRow<FMT, CONTIG, 2>;
-            const RowH even{yrow.base, yrow.tile_stride, yrow.shift, yrow.scale, yrow.half, 0};
-            const RowH odd{yrow.base, yrow.tile_stride, yrow.shift, yrow.scale, yrow.half, 1};
-            fft_pass<M, T, C::P, C::R0, 1, C::PADSHIFT, kFromInt8Sum>(sd, sx0, plo, phi, tid,
-                                                                     nullptr, qlo, qhi);
-            if (*abort_flag) return;   // nothing in flight: the next copy is not issued yet
-            fft_pass<M, T, C::P, C::R1, C::R0, C::PADSHIFT, kFromShared, true>(sd, nullptr, plo,
-                                                                              phi, tid, t2);
-            if constexpr (C::R1b > 1)
-                fft_pass<M, T, C::P, C::R1b, C::R0 * C::R1, C::PADSHIFT, kFromShared>(
-                    sd, nullptr, plo, phi, tid);
-            last_pass_store<MM, PLAN>(sd, plo, phi, qlo, qhi, even, tid);
-            fft_pass<M, T, C::P, C::R0, 1, C::PADSHIFT, kFromInt8Diff>(sd, sx0, plo, phi, tid,
-                                                                      nullptr, qlo, qhi);
-            // that pass ended with a barrier: every thread has read the frame
-            issue_next_into_buffer();
-            fft_pass<M, T, C::P, C::R1, C::R0, C::PADSHIFT, kFromShared, true>(sd, nullptr, plo,
-                                                                              phi, tid, t2);
-            if constexpr (C::R1b > 1)
-                fft_pass<M, T, C::P, C::R1b, C::R0 * C::R1, C::PADSHIFT, kFromShared>(
-                    sd, nullptr, plo, phi, tid);
-            last_pass_store_odd<MM, PLAN>(sd, plo, phi, qlo, qhi, *odd_shift, odd, tid);
-            continue;
-        }
 
         if (a.pmask != nullptr) {
             // Lost packets count as zeros: clear them in the landed copy before
@@ -905,22 +770,22 @@ __global__ void __launch_bounds__(FeCfg<MM, PLAN, HALF>::T, FeCfg<MM, PLAN, HALF
     }
 }
 
-template <int MM, int PLAN, int FMT, bool CONTIG, bool HALF>
+template <int MM, int PLAN, int FMT, bool CONTIG>
 corr_status launch_one(const FengineArgs &a, const TwiddleTables &tw, int num_sms,
                        cudaStream_t stream) {
-    using C = FeCfg<MM, PLAN, HALF>;
+    using C = FeCfg<MM, PLAN>;
     // Shared-memory limit and residency are per device: set up once on each.
     static PerDevice setup;
     static int per_sm[kMaxDeviceOrdinals];
     corr_status st = setup.run([](int dev) {
         corr_status s2 = cuda_check(
-            cudaFuncSetAttribute(fengine_kernel<MM, PLAN, FMT, CONTIG, HALF>,
+            cudaFuncSetAttribute(fengine_kernel<MM, PLAN, FMT, CONTIG>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM),
             "cudaFuncSetAttribute(fengine)");
         if (s2 != CORR_OK) return s2;
         int blocks = 0;
         s2 = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                            &blocks, fengine_kernel<MM, PLAN, FMT, CONTIG, HALF>, C::T, C::SMEM),
+                            &blocks, fengine_kernel<MM, PLAN, FMT, CONTIG>, C::T, C::SMEM),
                         "cudaOccupancyMaxActiveBlocksPerMultiprocessor(fengine)");
         if (s2 != CORR_OK) return s2;
         if (blocks < 1)
@@ -936,23 +801,23 @@ corr_status launch_one(const FengineArgs &a, const TwiddleTables &tw, int num_sm
     int grid = num_sms * per_sm[dev];
     if (grid > items) grid = items;
     TwPtrs p{tw.pass_lo, tw.pass_hi, tw.post_lo, tw.post_hi, tw.odd_shift};
-    fengine_kernel<MM, PLAN, FMT, CONTIG, HALF><<<grid, C::T, C::SMEM, stream>>>(a, p);
+    fengine_kernel<MM, PLAN, FMT, CONTIG><<<grid, C::T, C::SMEM, stream>>>(a, p);
     return cuda_check(cudaGetLastError(), "fengine_kernel launch");
 }
 
-template <int MM, int PLAN, bool HALF = false>
+template <int MM, int PLAN>
 corr_status launch_plan(const FengineArgs &a, const TwiddleTables &tw, int num_sms,
                         cudaStream_t stream) {
-    const bool contig = a.ytile == (HALF ? 2 * MM : MM);
+    const bool contig = a.ytile == MM;
     if (a.y_fmt == kSpectraF16)
-        return contig ? launch_one<MM, PLAN, kSpectraF16, true, HALF>(a, tw, num_sms, stream)
-                      : launch_one<MM, PLAN, kSpectraF16, false, HALF>(a, tw, num_sms, stream);
+        return contig ? launch_one<MM, PLAN, kSpectraF16, true>(a, tw, num_sms, stream)
+                      : launch_one<MM, PLAN, kSpectraF16, false>(a, tw, num_sms, stream);
     if (a.y_fmt == kSpectraF16Split)
-        return contig ? launch_one<MM, PLAN, kSpectraF16Split, true, HALF>(a, tw, num_sms, stream)
-                      : launch_one<MM, PLAN, kSpectraF16Split, false, HALF>(a, tw, num_sms,
+        return contig ? launch_one<MM, PLAN, kSpectraF16Split, true>(a, tw, num_sms, stream)
+                      : launch_one<MM, PLAN, kSpectraF16Split, false>(a, tw, num_sms,
                                                                             stream);
-    if (contig) return launch_one<MM, PLAN, kSpectraF32, true, HALF>(a, tw, num_sms, stream);
-    return launch_one<MM, PLAN, kSpectraF32, false, HALF>(a, tw, num_sms, stream);
+    if (contig) return launch_one<MM, PLAN, kSpectraF32, true>(a, tw, num_sms, stream);
+    return launch_one<MM, PLAN, kSpectraF32, false>(a, tw, num_sms, stream);
 }
 
 template <int MM>
@@ -961,21 +826,6 @@ corr_status launch_size(const FengineArgs &a, const TwiddleTables &tw, int num_s
     if (a.fplan != 0)
         return failf(CORR_ERR_ARG, "FFT plan %d is not available at n_freq=%d", a.fplan, MM);
     return launch_plan<MM, 0>(a, tw, num_sms, stream);
-}
-
-// n_freq = 2*MH above 16384: two MH-point transforms per frame.
-template <int MH>
-corr_status launch_half(const FengineArgs &a, const TwiddleTables &tw, int num_sms,
-                        cudaStream_t stream) {
-    if (a.fplan != 0)
-        return failf(CORR_ERR_ARG, "FFT plan %d is not available at n_freq=%d", a.fplan, 2 * MH);
-    if (a.pmask != nullptr)
-        return failf(CORR_ERR_ARG,
-                     "n_freq=%d: packet masks cover frames of at most 32 packets (n_freq <= 16384)",
-                     2 * MH);
-    if (tw.odd_shift == nullptr)
-        return failf(CORR_ERR_INTERNAL, "n_freq=%d: twiddle tables lack the odd-bin shift", 2 * MH);
-    return launch_plan<MH, 0, true>(a, tw, num_sms, stream);
 }
 
 } // namespace

@@ -106,23 +106,32 @@ constexpr int inverse_mod(int a, int m) {
     return x;
 }
 
-// Radix 4 x R2 or 8 x R2 with an odd R2, prime-factor form (no twiddles): input n =
+// Radix 2, 4 or 8 x R2 with an odd R2, prime-factor form (no twiddles): input n =
 // (R2 n1 + R1 n2) mod R, output k = (R2 (R2^-1 mod R1) k1 + R1 (R1^-1 mod R2) k2) mod
-// R. The inputs carry the int8 unpacking's offset (Dft<4>::run_biased).
+// R. BIASED inputs carry the int8 unpacking's offset (Dft<4>::run_biased).
 template <int R1, int R2>
 struct DftPfa {
     static constexpr int R = R1 * R2;
     static constexpr int U1 = R2 * inverse_mod(R2, R1), U2 = R1 * inverse_mod(R1, R2);
-    static __device__ __forceinline__ void run(float2 *v, float2 two_b) {
+    template <bool BIASED>
+    static __device__ __forceinline__ void run(float2 *v, float2 two_b = float2{}) {
+        static_assert(R1 > 2 || !BIASED, "radix 2 takes plain inputs");
         float2 y[R2][R1];
 #pragma unroll
         for (int n2 = 0; n2 < R2; ++n2) {
 #pragma unroll
             for (int n1 = 0; n1 < R1; ++n1) y[n2][n1] = v[(R2 * n1 + R1 * n2) % R];
-            if constexpr (R1 == 4)
+            if constexpr (R1 == 2) {
+                const float2 s = cadd(y[n2][0], y[n2][1]);
+                y[n2][1] = csub(y[n2][0], y[n2][1]);
+                y[n2][0] = s;
+            } else if constexpr (R1 == 4 && BIASED) {
                 Dft<4>::run_biased(y[n2], two_b);
-            else
-                Dft<R1>::template run<true>(y[n2], two_b);
+            } else if constexpr (R1 == 4) {
+                Dft<4>::run(y[n2]);
+            } else {
+                Dft<R1>::template run<BIASED>(y[n2], two_b);
+            }
         }
 #pragma unroll
         for (int k1 = 0; k1 < R1; ++k1) {
@@ -140,9 +149,9 @@ template <int R>
 __device__ __forceinline__ void dft_from_int8(float2 *v) {
     const float2 two_b = make_float2(2.0f * kInt8Bias, 2.0f * kInt8Bias);
     if constexpr (R == 12 || R == 20 || R == 28)
-        DftPfa<4, R / 4>::run(v, two_b);
+        DftPfa<4, R / 4>::template run<true>(v, two_b);
     else if constexpr (R == 24)
-        DftPfa<8, 3>::run(v, two_b);
+        DftPfa<8, 3>::run<true>(v, two_b);
     else
         Dft<R>::template run<true>(v, two_b);
 }

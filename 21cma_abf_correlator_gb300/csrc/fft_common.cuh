@@ -68,6 +68,7 @@ struct YRow {
     float scale;
     float half;            // scale / 2
     int odd = 0;           // STEP 2: 0 = even bins, 1 = odd bins
+    uint64_t policy = 0;   // STEP 2, 8-byte bins: L2 eviction policy of the stores
     __device__ __forceinline__ void put(int k, float2 v) const {
         if constexpr (STEP == 2) k = 2 * k + odd;
         T *dst = CONTIG ? base + k
@@ -80,8 +81,18 @@ struct YRow {
             const __half2 h = __floats2half2_rn(x, y);
             const float2 hf = __half22float2(h);
             const __half2 l = __floats2half2_rn(x - hf.x, y - hf.y);
-            *dst = make_uint2(*reinterpret_cast<const uint32_t *>(&h),
-                              *reinterpret_cast<const uint32_t *>(&l));
+            const uint2 hl = make_uint2(*reinterpret_cast<const uint32_t *>(&h),
+                                        *reinterpret_cast<const uint32_t *>(&l));
+            if constexpr (STEP == 2)
+                asm volatile("st.global.L2::cache_hint.v2.b32 [%0], {%1, %2}, %3;" ::"l"(dst),
+                             "r"(hl.x), "r"(hl.y), "l"(policy)
+                             : "memory");
+            else
+                *dst = hl;
+        } else if constexpr (STEP == 2) {
+            asm volatile("st.global.L2::cache_hint.v2.f32 [%0], {%1, %2}, %3;" ::"l"(dst),
+                         "f"(v.x), "f"(v.y), "l"(policy)
+                         : "memory");
         } else {
             *dst = v;
         }

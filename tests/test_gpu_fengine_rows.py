@@ -46,6 +46,14 @@ def test_ragged_counts_and_missing_frames(pkg, cuda, oracle, nf, n, frames):
         eng.close()
 
 
+@pytest.mark.parametrize("nf", [18432, 20480, 22528, 24576, 26624, 28672, 30720, 32768])
+@pytest.mark.parametrize("n,frames", [(1, 1), (1, 331)])   # 331: two or three a CTA
+def test_split_frames_missing(pkg, cuda, oracle, nf, n, frames):
+    """Above 16384 (two transforms a frame): the next frame is regrouped during the one
+    before, with frames missing in between."""
+    test_ragged_counts_and_missing_frames(pkg, cuda, oracle, nf, n, frames)
+
+
 @pytest.mark.parametrize("nf", [4096, 6144, 10240, 16384])
 def test_every_single_packet(pkg, cuda, oracle, nf):
     """Frame f keeps only packet f mod the frame's packets."""
