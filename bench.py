@@ -475,8 +475,8 @@ def main() -> None:
                 "alg_bytes_per_launch": dk["alg_bytes"], "frames_per_launch": PASS_FRAMES}
     if dom == "fengine":
         roofline["limiter"] = ("FP32 FFT arithmetic and shared-memory exchanges, not HBM: ncu on a "
-                               "256-frame launch saw the FP32 pipe 52 % busy, shared-memory "
-                               "wavefronts at 47 % and DRAM at 25 % of peak")
+                               "256-frame launch saw the FP32 pipe 57 % busy, shared-memory "
+                               "wavefronts at 48 % and DRAM at 30 % of peak")
 
     e2e = None
     if not args.no_e2e and rank == 0:
