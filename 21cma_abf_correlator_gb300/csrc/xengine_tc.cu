@@ -224,7 +224,12 @@ TcGeom make_geom(int n_station, bool split, int ct, int kt) {
     if (fixed + g.n_op * g.op_stage + 2 * g.ld_stage > budget) return g;
     // a third operand stage when it still leaves a four-deep load ring
     if (fixed + 3 * g.op_stage + 4 * g.ld_stage <= budget) g.n_op = 3;
-    g.n_ld = std::min(kMaxLoadStages, (budget - fixed - g.n_op * g.op_stage) / g.ld_stage);
+    // An even ring: each slot belongs to one converter group, which so has seen every
+    // earlier load of the slot land. In an odd one, a group could look at a slot whose
+    // load before, the other group's, is still in flight, and take the phase two loads
+    // back, which has the same parity, for its own.
+    g.n_ld = std::min(kMaxLoadStages, (budget - fixed - g.n_op * g.op_stage) / g.ld_stage) /
+             kConvGroups * kConvGroups;
     g.smem = g.n_ld * g.ld_stage + g.n_op * g.op_stage + fixed;
     // Two CTAs on one SM would both need more than half of TMEM and the second
     // would stall in tcgen05.alloc for the first's whole (persistent) life:
