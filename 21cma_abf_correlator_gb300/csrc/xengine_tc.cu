@@ -884,15 +884,20 @@ namespace corrgb {
 void xengine_tc_default_shape(int n_station, bool split, int *ct, int *kt) {
     // 32-frame stages halve the per-stage handoffs of 16-frame ones; then the
     // widest tile that fits.
+    // But not with a load ring of two, which leaves both converter groups waiting,
+    // where 16-frame stages fit one of four or more: 54 inputs, n_freq 4096, 1496
+    // frames, split form, F- and X-engine 1868 us at 32 frames, 1707 at 16.
     *ct = 0;
     *kt = 0;
     for (int k : {32, 16})
-        for (int c = 8; c >= 2; c /= 2)
-            if (make_geom(n_station, split, c, k).ok) {
-                *ct = c;
-                *kt = k;
-                return;
-            }
+        for (int c = 8; c >= 2; c /= 2) {
+            const TcGeom g = make_geom(n_station, split, c, k);
+            if (!g.ok) continue;
+            if (k == 32 && g.n_ld < 4 && make_geom(n_station, split, c, 16).n_ld >= 4) continue;
+            *ct = c;
+            *kt = k;
+            return;
+        }
 }
 
 corr_status xengine_tc_launch(const XengineArgs &a, bool split, int ct, int kt, int num_sms,
