@@ -220,8 +220,10 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
                     const int nf = MASK == 0 && KIND != kAny ? 0 : min(p.fs, n_left);
 #pragma unroll 1
                     for (int f = 0; f < nf; f += 2, xj += step) {
-                        // the odd frame of a last pair, which is not there, counts as zeros
-                        const float2 *yk = f + half < nf ? xj + to_k : zeros + lane_off;
+                        // the odd frame of a last pair, which is not there, counts as
+                        // zeros; zeros has one station after the other, whatever the
+                        // layout of the ring (ch + (kTile - 1) * rs stays inside it)
+                        const float2 *yk = f + half < nf ? xj + to_k : zeros + ch;
                         constexpr int NY = MASK == 0x5 || MASK == 0x1 ? kSub : kTile;
                         constexpr int NX = MASK == 0x1 ? kSub : kTile;
                         float2 x[kTile], y[kTile];

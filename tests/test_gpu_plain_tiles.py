@@ -81,3 +81,31 @@ def test_few_tiles_of_long_rows(pkg, cuda, oracle):
         pkg.set_device_map(None)
     assert oracle.normalized_max_err(one, oracle.correlate_rows(x, frames), n) < 1e-5
     assert split.tobytes() == one.tobytes()
+
+
+@pytest.mark.parametrize("acc64", [False, True], ids=["fp32rows", "fp64rows"])
+@pytest.mark.parametrize("n,nf,frames", [(n, 1024, f) for n in (3, 7, 24) for f in (1, 9, 33, 257)] +
+                         [(7, 32768, 9)])   # 32768: the frames are not summed in parts
+def test_odd_frame_counts_in_narrow_tiles(pkg, cuda, n, nf, frames, acc64):
+    """Spectra tiles narrower than the 16 channels of a warp, in launches whose last pair
+    of frames has only one: the layout moves data and changes no sum, so the rows are those
+    of contiguous spectra bit for bit."""
+    torch = cuda
+    rng = np.random.default_rng(100 * n + frames)
+    x = torch.from_numpy(rng.integers(-60, 61, size=(n, frames, 2 * nf)).astype(np.int8)).cuda()
+    eng = pkg.FxEngine(n, nf, max_frames=frames, xmode=0)
+    rows = {}
+    try:
+        if acc64:
+            eng.set_accumulator(pkg.abi.CORRX_ACC_FP64)
+        for ytile in (nf, 2, 4, 8):
+            eng.set_tiles(ytile)
+            rows[ytile] = eng.new_acc()
+            eng.accumulate(x, frames, rows[ytile])
+        torch.cuda.synchronize()
+        eng.check()
+    finally:
+        eng.close()
+    assert rows[nf].abs().max() > 0
+    for ytile in (2, 4, 8):
+        assert torch.equal(rows[ytile], rows[nf]), ytile
