@@ -198,7 +198,9 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
                 for (int l = 0; l < kTile; ++l) re[i][l] = im[i][l] = 0.f;
 
             // The round's frames, two a step, one per half warp: the sub-blocks of
-            // `mask`; on a tile of the diagonal (DIAG) the pairs k < j are left out.
+            // `mask`; on a tile of the diagonal (DIAG) the pairs k < j are left out. False,
+            // to the whole warp, once a wait has run out: its lanes leave together, as the
+            // shuffles and votes below take all of them.
             auto sum_frames = [&](auto mask_tag, auto diag_tag, int mask_arg) {
                 constexpr int MASK = decltype(mask_tag)::value;
                 constexpr bool DIAG = decltype(diag_tag)::value;
@@ -210,11 +212,12 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
                 int n_left = n_mine;
                 for (int s = round_stages(r); s > 0; --s, n_left -= p.fs, ++used) {
                     const int slot = used & slot_mask;
-                    if (!mbar_wait_bounded(&full[slot],
-                                           static_cast<uint32_t>(used >> p.slot_shift) & 1u, p.err,
-                                           kErrXengineMmaTimeout, abort_flag)) {
+                    const bool landed = mbar_wait_bounded(
+                        &full[slot], static_cast<uint32_t>(used >> p.slot_shift) & 1u, p.err,
+                        kErrXengineMmaTimeout, abort_flag);
+                    if (!__all_sync(0xffffffffu, landed)) {
                         s_abort = 1;
-                        return;
+                        return false;
                     }
                     const float2 *xj = run + slot * slot_elems;
                     const int nf = MASK == 0 && KIND != kAny ? 0 : min(p.fs, n_left);
@@ -260,22 +263,24 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&empty[slot]);
                 }
+                return true;
             };
             using std::integral_constant;
+            bool summed;
             if (sub == 0xf) {
-                sum_frames(integral_constant<int, 0xf>{}, std::false_type{}, 0);
+                summed = sum_frames(integral_constant<int, 0xf>{}, std::false_type{}, 0);
             } else if (sub == 0xb && J == K) {   // a whole tile of the diagonal
-                sum_frames(integral_constant<int, 0xb>{}, std::true_type{}, 0);
+                summed = sum_frames(integral_constant<int, 0xb>{}, std::true_type{}, 0);
             } else if (KIND == kAny) {
-                sum_frames(integral_constant<int, 0>{}, std::false_type{}, sub);
+                summed = sum_frames(integral_constant<int, 0>{}, std::false_type{}, sub);
             } else if (KIND == kEdge && sub == 0x5) {   // the last column, of 1 to 3 stations
-                sum_frames(integral_constant<int, 0x5>{}, std::false_type{}, 0);
+                summed = sum_frames(integral_constant<int, 0x5>{}, std::false_type{}, 0);
             } else if (KIND == kEdge && sub == 0x1) {   // and its diagonal tile
-                sum_frames(integral_constant<int, 0x1>{}, std::true_type{}, 0);
+                summed = sum_frames(integral_constant<int, 0x1>{}, std::true_type{}, 0);
             } else {   // no tile: the slots only pass
-                sum_frames(integral_constant<int, 0>{}, std::false_type{}, 0);
+                summed = sum_frames(integral_constant<int, 0>{}, std::false_type{}, 0);
             }
-            if (s_abort) return;
+            if (!summed) return;
             if (sub == 0) continue;
 
             // The half warps' sums together (even + odd frames), each half warp
@@ -287,13 +292,13 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
                 const long long t0 = clock64();
                 bool mine = true;
                 while (*turn != t) {
-                    if (s_abort || clock64() - t0 > kWaitBudgetCycles) {
+                    if (*abort_flag != 0 || clock64() - t0 > kWaitBudgetCycles) {
                         mine = false;
                         break;
                     }
                 }
                 if (!__all_sync(0xffffffffu, mine)) {
-                    if (p.err != nullptr && s_abort == 0) atomicExch(p.err, kErrXengineMmaTimeout);
+                    if (p.err != nullptr && *abort_flag == 0) atomicExch(p.err, kErrXengineMmaTimeout);
                     s_abort = 1;
                     return;
                 }
