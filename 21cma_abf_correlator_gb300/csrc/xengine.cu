@@ -53,7 +53,7 @@ constexpr int kMaxWarps = 15; // summing warps per CTA; one more loads
 constexpr int kMaxSlots = 8;  // TMA ring depth, at most
 constexpr int kMaxParts = 8;  // runs of frames summed apart, at most
 constexpr int kSumElems = kTile * kSub * 32;   // float2 of a tile's sum
-constexpr int kMaxTiles = 253;   // 22 x 22 / 2 tiles of 128 stations
+constexpr int kMaxTiles = 253;   // 22 x 23 / 2 tiles of 128 stations
 
 // Which tiles a launch has: whole ones only; whole ones and, in the last column,
 // ones of at most kSub stations (n_station % kTile = 1 .. 3); any (some baselines
@@ -161,13 +161,12 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
                     }
                 }
             }
-            // An aborted CTA lets every load in flight land before it exits. (One
-            // that ran through has read them all.)
-            if (!ok)
-                for (int s = 0; s <= slot_mask; ++s) {
-                    const uint32_t n_s = static_cast<uint32_t>(n + slot_mask - s) >> p.slot_shift;
-                    if (n_s > 0) mbar_wait_bounded(&full[s], (n_s - 1) & 1u, nullptr, 0);
-                }
+            // Every load lands before this thread leaves, and with it the CTA's shared
+            // memory, also where the summing warps have given up on the last ones.
+            for (int s = 0; s <= slot_mask; ++s) {
+                const uint32_t n_s = static_cast<uint32_t>(n + slot_mask - s) >> p.slot_shift;
+                if (n_s > 0) mbar_wait_bounded(&full[s], (n_s - 1) & 1u, nullptr, 0);
+            }
         }
         return;
     }
