@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (ok && op_lap > 0)
                 ok = mbar_wait_bounded(&bars.op_empty[ob], (op_lap - 1) & 1u, p.err,
                                        kErrXengineMmaTimeout, abort_flag);
-            if (!ok) {
+            if (!__all_sync(0xffffffffu, ok)) {   // the warp leaves together
                 s_abort = 1;
                 break;
             }
@@ -667,10 +667,17 @@ __global__ void __launch_bounds__(kThreads, 1)
         // warp (consecutive j) store to consecutive addresses:
         //   Vt[c][k(k+1)/2 + j] = V[j][k] (j <= k),  Qs[c][k][j] = Q[j][k].
         const int plane_v = n_baseline;
+        // A wait's outcome, one for the warp: its lanes leave together, as the tensor
+        // memory loads, shuffles and warp barriers between the waits take all of them.
+        auto warp_wait = [&](uint64_t *bar, uint32_t parity) {
+            const bool ok =
+                mbar_wait_bounded(bar, parity, p.err, kErrXengineMmaTimeout, abort_flag);
+            return __all_sync(0xffffffffu, ok) != 0;
+        };
         for (int tl = 0; tl < my_tiles; ++tl) {
             const int aset = g.n_acc == 2 ? tl & 1 : 0;
             const int acc_lap = g.n_acc == 2 ? tl >> 1 : tl;
-            if (!mbar_wait_bounded(&bars.acc_full[aset], static_cast<uint32_t>(acc_lap) & 1u, p.err, kErrXengineMmaTimeout, abort_flag)) {
+            if (!warp_wait(&bars.acc_full[aset], static_cast<uint32_t>(acc_lap) & 1u)) {
                 s_abort = 1;
                 break;
             }
@@ -738,7 +745,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 mbar_arrive(&bars.acc_empty[aset]);
                 mbar_arrive(&bars.epi);
             }
-            if (!mbar_wait_bounded(&bars.epi, 0u, p.err, kErrXengineMmaTimeout, abort_flag)) {
+            if (!warp_wait(&bars.epi, 0u)) {
                 s_abort = 1;
                 break;
             }
@@ -787,7 +794,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             // everyone done with Vs/Qs before the next tile overwrites them
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars.epi);
-            if (!mbar_wait_bounded(&bars.epi, 1u, p.err, kErrXengineMmaTimeout, abort_flag)) {
+            if (!warp_wait(&bars.epi, 1u)) {
                 s_abort = 1;
                 break;
             }
