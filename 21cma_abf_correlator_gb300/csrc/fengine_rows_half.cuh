@@ -311,6 +311,7 @@ __global__ void __launch_bounds__(512, 1) fengine_rows_half_kernel(FengineArgs a
             __syncwarp();
             if (lane == 0) mbar_arrive(data_read);
             if (odd) {
+                __syncwarp();   // the loads take the whole warp
 #pragma unroll
                 for (int c = 0; c < R / 8; ++c) {
                     float2 w[8];
