@@ -889,20 +889,29 @@ extern "C" corr_status corrx_tc_geometry(int32_t n_station, int32_t split, int32
 namespace corrgb {
 
 void xengine_tc_default_shape(int n_station, bool split, int *ct, int *kt) {
-    // 32-frame stages halve the per-stage handoffs of 16-frame ones; then the
-    // widest tile that fits.
-    // But not with a load ring of two, which leaves both converter groups waiting,
-    // where 16-frame stages fit one of four or more: 54 inputs, n_freq 4096, 1496
-    // frames, split form, F- and X-engine 1868 us at 32 frames, 1707 at 16.
+    // 32-frame stages halve the per-stage handoffs of 16-frame ones; then the widest tile
+    // that fits. But a load ring of two leaves both converter groups waiting. Then the next
+    // narrower tile, as long as its pieces stay at 32 bytes; 16-byte ones are bound by their
+    // number, and 16-frame stages of the same width are the faster ones. X-engine, split
+    // form, n_freq 16384, 512 frames (us; only split shapes have a ring of two):
+    //   inputs  16: 8 x 32 259, 4 x 32 242, 8 x 16 274    18: 356, 245, 379
+    //   inputs  30: 4 x 32 507, 2 x 32 469, 4 x 16 415    32: 543, 497, 428
+    //   inputs  54: 2 x 32 1440, 2 x 16 1221              62: 1581, 1421
     *ct = 0;
     *kt = 0;
     for (int k : {32, 16})
         for (int c = 8; c >= 2; c /= 2) {
             const TcGeom g = make_geom(n_station, split, c, k);
             if (!g.ok) continue;
-            if (k == 32 && g.n_ld < 4 && make_geom(n_station, split, c, 16).n_ld >= 4) continue;
             *ct = c;
             *kt = k;
+            if (k == 32 && g.n_ld < 4) {
+                const TcGeom narrow = make_geom(n_station, split, c / 2, 32);
+                if (narrow.ok && narrow.n_ld >= 4 && c / 2 * narrow.elem >= 32)
+                    *ct = c / 2;
+                else if (make_geom(n_station, split, c, 16).n_ld >= 4)
+                    *kt = 16;
+            }
             return;
         }
 }

@@ -184,3 +184,18 @@ def test_unknown_fft_plan_is_refused(pkg, cuda):
             eng.set_tiles(t["ytile"], t["xct"], t["xkt"], -1)
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("xmode,n,ct,kt", [
+    (2, 13, 8, 32), (2, 14, 4, 32), (2, 19, 4, 32), (2, 24, 4, 32), (2, 29, 4, 32),
+    (2, 30, 4, 16), (2, 32, 4, 16), (2, 33, 2, 32), (2, 52, 2, 32), (2, 53, 2, 16),
+    (2, 64, 2, 16), (1, 28, 8, 32), (1, 29, 4, 32), (1, 56, 4, 32), (1, 57, 4, 16)])
+def test_default_tensor_tile(pkg, cuda, xmode, n, ct, kt):
+    """The tile an engine that was not tuned takes: 32-byte pieces where they fit, a load
+    ring of four stages or more."""
+    eng = pkg.FxEngine(n, 512, max_frames=16, xmode=xmode)
+    try:
+        t = eng.tiles()
+    finally:
+        eng.close()
+    assert (t["xct"], t["xkt"]) == (ct, kt)
