@@ -340,15 +340,12 @@ __global__ void __launch_bounds__(512, 1) fengine_rows_kernel(FengineArgs a, TwP
     issue(cur);
     int nxt = n_items;
     if (cur < n_items) {
-        deinterleave(cur, 1);   // word 1: frame 0's waits may already be setting word 0
+        deinterleave(cur, 0);
         nxt = next_present(cur + stride);
         meet();
-        if (abort_flag[1]) {   // no second copy on a barrier whose first has not landed
-            if (t == 0) mbar_wait_bounded(bar, 0, nullptr, 0);
-            cur = n_items;
-        } else {
-            issue(nxt);
-        }
+        // no second copy on a barrier whose first has not landed: leave at frame 0's meeting
+        if (abort_flag[0]) nxt = n_items;
+        issue(nxt);
     }
     float2 *const drow = sd + wf * RPW * C::DROW;     // this warp's rows
     // second pass: lane = row and k1 (the lanes past RPW*R0 repeat lane 0's work)
@@ -416,8 +413,8 @@ __global__ void __launch_bounds__(512, 1) fengine_rows_kernel(FengineArgs a, TwP
             }
         }
         meet();
-        if (abort_flag[n & 1]) {   // let the copy in flight, if any, land
-            if (t == 0 && nxt < n_items) mbar_wait_bounded(bar, parity ^ 1u, nullptr, 0);
+        if (abort_flag[n & 1]) {   // let the copy last waited for land
+            if (t == 0) mbar_wait_bounded(bar, parity ^ 1u, nullptr, 0);
             break;
         }
         const int after = next_present(nxt + stride);
