@@ -205,7 +205,7 @@ corr_status fengine_launch(int n_freq, const TwiddleTables &tw, const FengineArg
 corr_status xengine_plain_launch(const XengineArgs &a, int num_sms, cudaStream_t stream);
 /// The plain X-engine's tiles of 6 x 6 stations, each with the mask of its 3 x 3
 /// sub-blocks, that hold the given baselines (ascending indices of the row-major
-/// numbering j <= k; empty: all of them).
+/// numbering j <= k).
 void xengine_plain_tiles(int n_station, const std::vector<int32_t> &baselines,
                          std::vector<uint16_t> *out);
 corr_status scale_launch(float2 *acc, size_t n, float s, cudaStream_t stream);
