@@ -602,31 +602,51 @@ corr_status xengine_plain_launch(const XengineArgs &a, int num_sms, cudaStream_t
     };
     // CTA shape: every tile of a channel tile if they fit, in tile groups (that
     // read the same spectra) otherwise; then parts side by side; then channel
-    // tiles, as long as each SM still gets a CTA. Not wider than the ring has room
-    // for (a few baselines of many stations: few tiles, long runs).
+    // tiles. Not wider than the ring has room for (a few baselines of many
+    // stations: few tiles, long runs).
     p.tile_groups = (p.n_tiles + kMaxWarps - 1) / kMaxWarps;
     p.tiles = (p.n_tiles + p.tile_groups - 1) / p.tile_groups;
     p.slots_p = 1;
     while (p.slots_p < p.n_parts && p.tiles * p.slots_p * 2 <= kMaxWarps &&
            budget_of(p.slots_p * 2, 1, 1) > 0)
         p.slots_p *= 2;
-    p.slots_c = 1;
-    while (p.tiles * p.slots_p * (p.slots_c + 1) <= kMaxWarps &&
-           (n_ct + p.slots_c) / (p.slots_c + 1) * p.tile_groups >= num_sms &&
-           budget_of(p.slots_p, p.slots_c + 1, 1) > 0)
-        ++p.slots_c;
+    // Channel tiles side by side: as many as cost least. The busiest SM's tiles take
+    // about their frames and 10 more for each part; every round of a CTA's units takes
+    // another 100, since its first loads and its last sums have nothing beside them.
+    // (100 and 10 come within 1.5 % of the best width over 550 launches: 1 to 40
+    // stations, n_freq 1024 to 32768, 1 to 512 frames.) As wide as leaves each SM a
+    // CTA, which was the rule, left a second round nearly empty: n_freq 32768, 4 stations
+    // 64 frames 54 -> 25 us, 1 station 4 frames 10.2 -> 6.0.
+    const int sms = std::max(1, num_sms);
+    int per_sm = 1;
+    int64_t least = -1;
+    for (int c = 1; p.tiles * p.slots_p * c <= kMaxWarps; ++c) {
+        int ctas = (kMaxWarps + 1) / (p.tiles * p.slots_p * c + 1);
+        while (ctas > 1 && budget_of(p.slots_p, c, ctas) == 0) --ctas;
+        if (budget_of(p.slots_p, c, ctas) == 0) break;
+        const int units = (n_ct + c - 1) / c * p.tile_groups;
+        const int rounds = (units + sms * ctas - 1) / (sms * ctas) * (p.n_parts / p.slots_p);
+        const int64_t busiest = static_cast<int64_t>((units + sms - 1) / sms) * c * p.tiles;
+        const int64_t cost = 100 * rounds + busiest * (10 * p.n_parts + a.frames);
+        // as dear, the narrower; but the wider with six tiles or more, whose warps CTA by
+        // CTA do not divide by the four schedulers (13 stations, n_freq 32768, 128 frames
+        // 1.15 times as long)
+        if (least >= 0 && (cost > least || (cost == least && p.tiles < 6))) continue;
+        least = cost;
+        per_sm = ctas;
+        p.slots_c = c;
+    }
+    if (least < 0)
+        return failf(CORR_ERR_ARG, "plain X-engine: %d stations do not fit in shared memory", N);
     p.units = (n_ct + p.slots_c - 1) / p.slots_c * p.tile_groups;
     place_tiles(tiles, &p);
     const size_t per_pair = run_pair * p.slots_p * p.slots_c;
     const int warps = p.tiles * p.slots_p * p.slots_c + 1;
-    int per_sm = std::max(1, (kMaxWarps + 1) / warps);
-    while (per_sm > 1 && budget_of(p.slots_p, p.slots_c, per_sm) == 0) --per_sm;
     const size_t budget = budget_of(p.slots_p, p.slots_c, per_sm);
-    if (budget == 0)
-        return failf(CORR_ERR_ARG, "plain X-engine: %d stations do not fit in shared memory", N);
     const size_t sums = p.n_parts > 1 ? p.tiles * p.slots_c * kSumElems * sizeof(float2) : 0;
     p.slot_shift = 8 * 16 * per_pair <= budget ? 3 : 2;
     p.fs = 2 * static_cast<int>(std::min<size_t>(16, (budget >> p.slot_shift) / per_pair));
+    p.fs = std::min(p.fs, p.seg);   // no stages longer than a part: their rest would be zeros
     const size_t ring = ((per_pair * (p.fs / 2)) << p.slot_shift) + pad;
     p.sums_at = static_cast<int>(ring / sizeof(float2));
     const size_t smem = ring + sums;
@@ -676,7 +696,7 @@ corr_status xengine_plain_launch(const XengineArgs &a, int num_sms, cudaStream_t
         return CORR_OK;
     });
     if (st != CORR_OK) return st;
-    const int grid = std::min(p.units, std::max(1, num_sms) * per_sm);
+    const int grid = std::min(p.units, sms * per_sm);
     const int kind = a.tiles != nullptr ? kAny : (N - 1) % kTile < kSub ? kEdge : kWhole;
     const Kernel kernel = kernels[(a.ytile >= kXch ? 0 : 3) + kind];
     kernel<<<grid, warps * 32, smem, stream>>>(map, p);
