@@ -77,7 +77,6 @@ struct PlainParams {
     int units;            // channel-tile groups x tile_groups
     int sums_at;          // float2 before the tiles' sums in shared memory
     void *acc;
-    int acc64;
     int *err;
     // J | K << 5 | sub-block mask << 10, groups of `tiles` one after the other (bit
     // 2a + b of the mask: blocks of kSub stations 2J + a, 2K + b); mask 0: no tile
@@ -86,8 +85,11 @@ struct PlainParams {
 
 // ROW: a run of frames in the ring holds [frame][station][16 channels] (ytile >= 16);
 // otherwise [spectra tile][frame][station][ytile], as the TMA box brings narrower tiles.
-// KIND: which tiles a launch has (kWhole, kEdge, kAny below).
-template <bool ROW, int KIND>
+// KIND: which tiles a launch has (kWhole, kEdge, kAny below). ACC64: complex128 rows.
+// A launch of few frames is bound by its instruction fetches, and both kinds of rows in
+// one kernel made the epilogue half as long again: 20 stations, n_freq 14336, 1 frame
+// 23.4 -> 17.2 us, 64 frames 95.7 -> 85.4 us.
+template <bool ROW, int KIND, bool ACC64>
 __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
     xengine_plain_kernel(const __grid_constant__ CUtensorMap ymap,
                          const __grid_constant__ PlainParams p) {
@@ -327,7 +329,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
                     const int k = K * kTile + l;
                     if (j <= k && k < N && ((sub >> (2 * half + l / kSub)) & 1)) {
                         const size_t at = row + static_cast<size_t>(k) * p.n_freq;
-                        if (p.acc64) {   // complex128 row: the FP32 sums added in double
+                        if constexpr (ACC64) {   // complex128 row: the FP32 sums added in double
                             double *dst = static_cast<double *>(p.acc) + 2 * at;
                             red_add_f64(dst, widen(v.x));
                             red_add_f64(dst + 1, widen(v.y));
@@ -655,7 +657,6 @@ corr_status xengine_plain_launch(const XengineArgs &a, int num_sms, cudaStream_t
     p.frames = a.frames;
     p.ytile = a.ytile;
     p.acc = a.acc;
-    p.acc64 = a.acc64;
     p.err = a.err;
 
     EncodeTiledFn enc = encode_tiled();
@@ -680,10 +681,13 @@ corr_status xengine_plain_launch(const XengineArgs &a, int num_sms, cudaStream_t
         return failf(CORR_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", static_cast<int>(cr));
 
     using Kernel = void (*)(CUtensorMap, PlainParams);
-    static constexpr Kernel kernels[6] = {
-        xengine_plain_kernel<true, kWhole>, xengine_plain_kernel<true, kEdge>,
-        xengine_plain_kernel<true, kAny>,   xengine_plain_kernel<false, kWhole>,
-        xengine_plain_kernel<false, kEdge>, xengine_plain_kernel<false, kAny>};
+    static constexpr Kernel kernels[12] = {
+        xengine_plain_kernel<true, kWhole, false>,  xengine_plain_kernel<true, kEdge, false>,
+        xengine_plain_kernel<true, kAny, false>,    xengine_plain_kernel<false, kWhole, false>,
+        xengine_plain_kernel<false, kEdge, false>,  xengine_plain_kernel<false, kAny, false>,
+        xengine_plain_kernel<true, kWhole, true>,   xengine_plain_kernel<true, kEdge, true>,
+        xengine_plain_kernel<true, kAny, true>,     xengine_plain_kernel<false, kWhole, true>,
+        xengine_plain_kernel<false, kEdge, true>,   xengine_plain_kernel<false, kAny, true>};
     static PerDevice setup;   // the shared-memory limit is a per-device setting
     corr_status st = setup.run([](int) {
         for (auto k : kernels) {
@@ -698,7 +702,7 @@ corr_status xengine_plain_launch(const XengineArgs &a, int num_sms, cudaStream_t
     if (st != CORR_OK) return st;
     const int grid = std::min(p.units, sms * per_sm);
     const int kind = a.tiles != nullptr ? kAny : (N - 1) % kTile < kSub ? kEdge : kWhole;
-    const Kernel kernel = kernels[(a.ytile >= kXch ? 0 : 3) + kind];
+    const Kernel kernel = kernels[(a.acc64 ? 6 : 0) + (a.ytile >= kXch ? 0 : 3) + kind];
     kernel<<<grid, warps * 32, smem, stream>>>(map, p);
     return cuda_check(cudaGetLastError(), "xengine_plain_kernel launch");
 }
