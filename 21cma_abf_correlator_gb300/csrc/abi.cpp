@@ -570,6 +570,7 @@ corr_status build_share(Context *c, Share &s, int home_physical) {
                             &s.plan)) != CORR_OK)
         return st;
     s.plan->acc64 = 1;
+    s.plan->run_stations = cfg.n_station;
     // A device of the baseline-range or pair-covering split owns only some
     // baselines of its stations' matrix: the plain X-engine computes only the
     // station-block pairs that hold them, so the devices divide its work.

@@ -98,7 +98,7 @@ corr_status fxplan_create(int device, int n_station, int n_freq, int max_frames,
     FxPlan *p = new (std::nothrow) FxPlan();
     if (p == nullptr) return fail(CORR_ERR_NOMEM, "fxplan_create: out of host memory");
     p->device = device;
-    p->n_station = n_station;
+    p->n_station = p->run_stations = n_station;
     p->n_freq = n_freq;
     p->n_baseline = n_station * (n_station + 1) / 2;
     p->max_frames = max_frames;
@@ -171,6 +171,7 @@ corr_status fxplan_accumulate(FxPlan *p, const int8_t *samples, size_t station_s
         fa.pmask_station_stride = pmask_station_stride;
         fa.pmask_frame0 = pmask_frame0 + f0;
         fa.n_station = p->n_station;
+        fa.run_stations = p->run_stations;
         fa.frames = ft;
         fa.y = p->d_y;
         fa.y_frames = p->max_frames;
@@ -361,6 +362,7 @@ extern "C" corr_status corrx_run_fengine(void *eng, const int8_t *d_samples,
     fa.mask_station_stride = mask_station_stride;
     fa.mask_bit0 = mask_bit0;
     fa.n_station = p->n_station;
+    fa.run_stations = p->run_stations;
     fa.frames = frames;
     fa.y = p->d_y;
     fa.y_frames = p->max_frames;

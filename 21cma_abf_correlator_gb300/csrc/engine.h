@@ -141,6 +141,7 @@ struct FengineArgs {
     size_t pmask_station_stride;
     int pmask_frame0;
     int n_station;
+    int run_stations;           // the run's, of which a device of a split holds n_station
     int frames;
     float2 *y;                  // spectra (y_index)
     int y_frames;               // frames the spectra buffer holds
@@ -247,6 +248,7 @@ struct FxPlan {
     int xkt = 0;          // tensor X-engine: frames per stage
     int fplan = 0;        // F-engine FFT radix plan
     int xmode = CORR_X_PLAIN_FP32;
+    int run_stations = 0; // the run's stations, of which a device of a split holds n_station
     int acc64 = 0;        // rows are complex128 (CORRX_ACC_FP64) instead of complex64
     std::vector<uint16_t> xtiles;   // plain X-engine: tiles to compute (empty: the whole matrix)
     int num_sms = 0;

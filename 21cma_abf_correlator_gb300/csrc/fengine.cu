@@ -30,7 +30,7 @@
 #include "fengine_impl.cuh"
 
 // This file: the host side (twiddle tables, plans, dispatch by length) and the
-// kernels of n_freq 512 .. 2048 and, for few frames, of 4096 .. 8192; fengine_impl.cuh
+// kernels of n_freq 512 .. 2048 and, for few transforms, of 4096 .. 8192; fengine_impl.cuh
 // holds the kernel templates, fengine_rows.cuh those of 4096 .. 16384, fengine_rows_half.cuh those above.
 
 namespace corrgb {
@@ -98,24 +98,27 @@ void fengine_release(TwiddleTables *tw) {
 
 corr_status fengine_launch(int n_freq, const TwiddleTables &tw, const FengineArgs &a,
                            int num_sms, cudaStream_t stream) {
+    const int64_t transforms = static_cast<int64_t>(a.frames) * a.run_stations;
     switch (n_freq) {
     case 512: return launch_size<512>(a, tw, num_sms, stream);
     case 1024: return launch_size<1024>(a, tw, num_sms, stream);
     case 2048: return launch_size<2048>(a, tw, num_sms, stream);
-    // The kernel of fengine_rows.cuh starts 2 us slower (its tensor-memory tables) and
-    // is faster per frame. 24 stations, FP16 output, old / rows: n_freq 4096 4 frames
-    // 6.9 / 9.0 us, 64 frames 18.9 / 21.1, 512 frames 115.2 / 109.8; n_freq 8192 4
-    // frames 8.5 / 10.7, 1024 frames 483 / 433. (From 10240 up it is the faster one
-    // from a few frames on: 12288 4 frames 12.7 / 13.0, 1024 frames 1115 / 900.) By
-    // frames alone, so that devices holding different stations take the same one.
+    // The kernel of fengine_rows.cuh takes 2 us longer for its first frame (tensor-memory
+    // tables, regrouped samples) and is faster per transform. FP16 output, this one /
+    // rows, by transforms: n_freq 4096 256: 5.4 / 7.6 us, 1600: 18.6 / 19.7, 6144: 59.1 /
+    // 57.9, 25600: 229 / 218; 6144 256: 9.0 / 10.7, 1024: 22.8 / 23.5, 1536: 34.1 / 33.3;
+    // 8192 256: 8.7 / 10.9, 1024: 22.9 / 24.2, 1536: 34.3 / 33.9, 25600: 501 / 463. The
+    // run's stations count, not the device's, so that devices holding different ones of
+    // them take the same kernel. (From 10240 up rows is the faster one from a few hundred
+    // transforms on, and 0.3 to 1.3 us the slower below: 16384 24: 9.2 / 10.5 us.)
     case 4096:
-        if (a.frames < 256) return launch_size<4096>(a, tw, num_sms, stream);
+        if (transforms < 6144) return launch_size<4096>(a, tw, num_sms, stream);
         return fengine_launch_rows_c(n_freq, tw, a, num_sms, stream);
     case 6144:
-        if (a.frames < 64) return launch_size<6144>(a, tw, num_sms, stream);
+        if (transforms < 1536) return launch_size<6144>(a, tw, num_sms, stream);
         return fengine_launch_rows_c(n_freq, tw, a, num_sms, stream);
     case 8192:
-        if (a.frames < 64) return launch_size<8192>(a, tw, num_sms, stream);
+        if (transforms < 1536) return launch_size<8192>(a, tw, num_sms, stream);
         return fengine_launch_rows_c(n_freq, tw, a, num_sms, stream);
     case 10240: case 12288: return fengine_launch_rows_b(n_freq, tw, a, num_sms, stream);
     case 14336: return fengine_launch_rows_a(n_freq, tw, a, num_sms, stream);

@@ -150,7 +150,7 @@ extern "C" corr_status corrx_accumulate_noalloc(int32_t n_station, int32_t n_fre
     fa.mask = d_mask;
     fa.mask_station_stride = mask_station_stride;
     fa.mask_bit0 = mask_bit0;
-    fa.n_station = n_station;
+    fa.n_station = fa.run_stations = n_station;
     fa.frames = frames;
     fa.y = d.spectra;
     fa.y_frames = frames;

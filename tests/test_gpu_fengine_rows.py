@@ -10,6 +10,8 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
+from abi_driver import drive_rows
+
 pytestmark = pytest.mark.gpu
 
 # stations x frames of 1 and 3 leave groups without a frame; 500 and 1201 are a few
@@ -79,15 +81,15 @@ def test_every_single_packet(pkg, cuda, oracle, nf):
     assert oracle.rel_rms(acc.cpu().numpy(), oracle.correlate(kept)) < 1e-5
 
 
-# Launches long enough for several frames to a CTA, each in its own group of warps:
-# n_freq 4096 from 256 frames on, 6144 and 8192 from 64. One station leaves groups without
-# a frame (256 and 64 frames are fewer than the GPU's groups), three go round several times.
-GROUPED = [(4096, 256), (4096, 301), (6144, 64), (6144, 101), (8192, 64), (8192, 203)]
+# Enough transforms for several frames to a CTA, each in its own group of warps: frames x
+# stations from 6144 on at n_freq 4096, from 1536 on at 6144 and 8192; one station and
+# several, whole rounds and ragged ones.
+GROUPED = [(4096, 1, 6144), (4096, 7, 901), (6144, 1, 1536), (6144, 7, 221), (8192, 1, 1537),
+           (8192, 5, 331)]
 
 
-@pytest.mark.parametrize("n", [1, 3])
-@pytest.mark.parametrize("nf,frames", GROUPED)
-def test_groups_with_packets_missing(pkg, cuda, oracle, nf, frames, n):
+@pytest.mark.parametrize("nf,n,frames", GROUPED)
+def test_groups_with_packets_missing(pkg, cuda, oracle, nf, n, frames):
     """Of station s, frame f keeps packet (f + s) mod the frame's packets alone; every
     fifth frame all of them, every seventh none."""
     torch = cuda
@@ -112,15 +114,15 @@ def test_groups_with_packets_missing(pkg, cuda, oracle, nf, frames, n):
 
 
 @pytest.mark.parametrize("xmode,ytile", [(0, 2), (0, 64), (1, 8), (2, 4)])
-@pytest.mark.parametrize("n", [1, 3])
-@pytest.mark.parametrize("nf,frames", GROUPED)
-def test_groups_in_channel_tiles(pkg, cuda, nf, frames, n, xmode, ytile):
-    """Spectra in channel tiles, frames missing: the rows of contiguous spectra bit for bit
-    (those against the oracle: test_ragged_counts_and_missing_frames)."""
+@pytest.mark.parametrize("nf,n,frames", GROUPED)
+def test_groups_in_channel_tiles(pkg, cuda, oracle, nf, n, frames, xmode, ytile):
+    """Frames missing; spectra in channel tiles give the rows of contiguous spectra bit for
+    bit, and the plain ones are the oracle's."""
     torch = cuda
     rng = np.random.default_rng(nf + frames + n)
-    x = torch.from_numpy(rng.integers(-100, 101, size=(n, frames, 2 * nf)).astype(np.int8)).cuda()
+    x = rng.integers(-100, 101, size=(n, frames, 2 * nf)).astype(np.int8)
     keep = rng.random((n, frames)) > 0.3
+    xs = torch.from_numpy(x).cuda()
     mask = torch.from_numpy(np.packbits(keep.astype(np.uint8), axis=1, bitorder="little")).cuda()
     eng = pkg.FxEngine(n, nf, max_frames=frames, xmode=xmode)
     rows = []
@@ -128,10 +130,28 @@ def test_groups_in_channel_tiles(pkg, cuda, nf, frames, n, xmode, ytile):
         for tiles in [(nf, 8, 16), (ytile, ytile, 16)]:
             eng.set_tiles(*tiles)
             rows.append(eng.new_acc())
-            eng.accumulate(x, frames, rows[-1], mask=mask)
+            eng.accumulate(xs, frames, rows[-1], mask=mask)
         torch.cuda.synchronize()
         eng.check()
     finally:
         eng.close()
-    assert rows[0].abs().max() > 0
     assert torch.equal(rows[0], rows[1])
+    if ytile == 2:
+        assert oracle.rel_rms(rows[0].cpu().numpy(), oracle.correlate(x, keep)) < 1e-5
+
+
+@pytest.mark.parametrize("nf,frames", [(4096, 256), (8192, 64)])
+def test_groups_without_a_frame(pkg, cuda, oracle, nf, frames):
+    """24 stations over eight devices by baseline range: each device has too few of the
+    run's frames for all of its groups, and takes the kernel that one device takes. The
+    rows are one device's, bit for bit."""
+    x = np.random.default_rng(nf).integers(-60, 61, size=(1, 24, frames, 2 * nf)).astype(np.int8)
+    one = drive_rows(pkg, x, frames, frames, chunk_frames=frames)
+    pkg.set_device_map([0] * 8)
+    try:
+        split = drive_rows(pkg, x, frames, frames, chunk_frames=frames, devices=list(range(8)),
+                           split_mode=0)
+    finally:
+        pkg.set_device_map(None)
+    assert oracle.normalized_max_err(one, oracle.correlate_rows(x, frames), 24) < 1e-5
+    assert split.tobytes() == one.tobytes()
