@@ -170,17 +170,27 @@ __device__ __forceinline__ void red_add_f64(double *dst, double v) {
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(gmem_addr(dst)), "d"(v) : "memory");
 }
 
-// {dst[0], dst[1]} += v in FP32, performed at L2, with no value returned.
+// {dst[0], dst[1]} += v in FP32, performed at L2, with no value returned; dst 8-byte
+// aligned. FP32 reductions take subnormal values of the row for zeros, so nothing is done
+// where v is zero (a station that is missing): they stay as they are. A v that is not
+// zero is far above them.
 __device__ __forceinline__ void red_add_f32x2(float2 *dst, float2 v) {
-    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(gmem_addr(dst)), "f"(v.x), "f"(v.y)
-                 : "memory");
+    if (v.x != 0.0f || v.y != 0.0f)
+        asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(gmem_addr(dst)), "f"(v.x),
+                     "f"(v.y)
+                     : "memory");
 }
 
-// dst[0..3] += {a.x, a.y, b.x, b.y} in FP32, likewise; dst 16-byte aligned.
+// dst[0..3] += {a.x, a.y, b.x, b.y} likewise; dst 16-byte aligned.
 __device__ __forceinline__ void red_add_f32x4(float2 *dst, float2 a, float2 b) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(gmem_addr(dst)), "f"(a.x),
-                 "f"(a.y), "f"(b.x), "f"(b.y)
-                 : "memory");
+    if ((a.x != 0.0f || a.y != 0.0f) && (b.x != 0.0f || b.y != 0.0f)) {
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(gmem_addr(dst)),
+                     "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y)
+                     : "memory");
+    } else {
+        red_add_f32x2(dst, a);
+        red_add_f32x2(dst + 1, b);
+    }
 }
 
 // (double)x in integer arithmetic. This GPU converts (and computes) doubles at

@@ -95,3 +95,36 @@ def test_abi_long_row_integrates_in_fp64(pkg, cuda, oracle, frames, reference):
     e_short = oracle.rel_rms(short[0], reference[SHORT])
     print(f"ABI rel RMS: {SHORT} frames {e_short:.2e}, {LONG} frames {e_long:.2e}")
     assert e_long < 1.5 * e_short + 1e-8 and e_long < 1e-6
+
+
+@pytest.mark.parametrize("acc64", [False, True], ids=["fp32rows", "fp64rows"])
+@pytest.mark.parametrize("xmode", [0, 1, 2])
+def test_missing_station_leaves_subnormal_rows(pkg, cuda, xmode, acc64):
+    """Adding nothing changes nothing: the baselines of a station without a frame keep the
+    subnormal values that a caller's row holds, bit for bit; the others are added to."""
+    torch = cuda
+    n, nf, frames = 7, 1024, 33
+    rng = np.random.default_rng(40)
+    x = torch.from_numpy(rng.integers(-60, 61, size=(n, frames, 2 * nf)).astype(np.int8)).cuda()
+    mask = torch.full((n, (frames + 7) // 8), 255, dtype=torch.uint8, device="cuda")
+    mask[2] = 0
+    eng = pkg.FxEngine(n, nf, max_frames=frames, xmode=xmode)
+    try:
+        if acc64:
+            eng.set_accumulator(pkg.abi.CORRX_ACC_FP64)
+        acc = eng.new_acc()
+        acc += (3e-310 - 1e-320j) if acc64 else (3e-40 - 1e-45j)
+        before = acc.cpu().numpy()
+        eng.accumulate(x, frames, acc, mask=mask)
+        torch.cuda.synchronize()
+        eng.check()
+        after = acc.cpu().numpy()
+    finally:
+        eng.close()
+    assert (before.real != 0).all() and (before.imag != 0).all()
+    b = 0
+    for j in range(n):
+        for k in range(j, n):
+            same = after[b].tobytes() == before[b].tobytes()
+            assert same == (2 in (j, k)), (j, k)
+            b += 1
