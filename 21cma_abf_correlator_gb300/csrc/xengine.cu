@@ -36,6 +36,7 @@
 //    4 inputs, n_freq  2048,  300 frames  0.093 -> 0.017 ms (64 one-warp CTAs before)
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 #include <vector>
 
@@ -449,12 +450,17 @@ __global__ void add64_kernel(double2 *__restrict__ dst, const double2 *__restric
     }
 }
 
-// (float)(v * s), s = s_hi + s_lo. This GPU multiplies and converts doubles at 2
-// lanes per SM and cycle, so v is cut, in integer arithmetic, into its leading 24
-// bits and the next 23 (exact to 2^-46 of v) and multiplied in FP32: the last FMA
-// rounds the product once, as the double one is rounded. Zeros, numbers near or past
-// FP32's range, infinities and NaN go the long way.
-__device__ __forceinline__ float scaled_to_float(double v, float s_hi, float s_lo, double s) {
+// (float)(v * s), s = s_hi + s_lo; exact: s is a power of two. This GPU multiplies and
+// converts doubles at 2 lanes per SM and cycle, so v is cut, in integer arithmetic, into
+// its leading 24 bits and the next 23 (and whether any bit follows) and multiplied in
+// FP32: hi * s_hi + tail, to 2^-44 of it, rounded once by the last FMA, as the double
+// product is rounded (exactly, if s is a power of two). Where 2^-43 more or less would
+// round another way, the double product decides. That happens once in 2^19 values; rows
+// that hold little else than ties (v a few bits longer than a float and s a power of two)
+// are the exact case. Zeros, numbers near or past FP32's range, infinities and NaN go the
+// long way too.
+__device__ __forceinline__ float scaled_to_float(double v, float s_hi, float s_lo, double s,
+                                                 bool exact) {
     const uint32_t top = static_cast<uint32_t>(__double2hiint(v));
     const uint32_t low = static_cast<uint32_t>(__double2loint(v));
     const uint32_t e = (top >> 20) & 0x7ffu;   // 1023 + exponent
@@ -467,7 +473,11 @@ __device__ __forceinline__ float scaled_to_float(double v, float s_hi, float s_l
     const float frac =
         __uint_as_float(0x3f800000u | ((low >> 6) & 0x7fffffu) | ((low & 0x3fu) != 0u)) - 1.0f;
     const float lo = frac * __uint_as_float(sign | (f_exp - (23u << 23)));
-    return fmaf(hi, s_hi, fmaf(hi, s_lo, lo * s_hi));
+    const float tail = fmaf(hi, s_lo, lo * s_hi);
+    const float r = fmaf(hi, s_hi, tail), d = fabsf(r) * 0x1p-43f;
+    const bool sure = exact || fmaf(hi, s_hi, tail + d) == fmaf(hi, s_hi, tail - d);
+    if (!sure || fabsf(r) < 0x1p-60f) return static_cast<float>(v * s);
+    return r;
 }
 
 // Two channels per thread and step: 32 bytes of complex128 in, 16 bytes of complex64
@@ -477,7 +487,7 @@ __global__ void __launch_bounds__(256)
     dump64_kernel(float2 *__restrict__ out, size_t out_row, const double2 *__restrict__ src,
                   size_t src_row, const int32_t *__restrict__ gmap,
                   const int32_t *__restrict__ lmap, int n_map, int half_freq, float s_hi,
-                  float s_lo, double s) {
+                  float s_lo, double s, bool exact) {
     const int r = blockIdx.x / n_map, m = blockIdx.x - r * n_map;
     const int gb = gmap ? gmap[m] : m;
     const int lb = lmap ? lmap[m] : m;
@@ -487,8 +497,10 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 2
     for (int c = blockIdx.y * 256 + threadIdx.x; c < half_freq; c += gridDim.y * 256) {
         const double2 a0 = a[2 * c], a1 = a[2 * c + 1];
-        o[c] = make_float4(scaled_to_float(a0.x, s_hi, s_lo, s), scaled_to_float(a0.y, s_hi, s_lo, s),
-                           scaled_to_float(a1.x, s_hi, s_lo, s), scaled_to_float(a1.y, s_hi, s_lo, s));
+        o[c] = make_float4(scaled_to_float(a0.x, s_hi, s_lo, s, exact),
+                           scaled_to_float(a0.y, s_hi, s_lo, s, exact),
+                           scaled_to_float(a1.x, s_hi, s_lo, s, exact),
+                           scaled_to_float(a1.y, s_hi, s_lo, s, exact));
     }
 }
 
@@ -827,8 +839,10 @@ corr_status dump64_launch(float2 *out, size_t out_row, const double2 *src, size_
     const dim3 grid(static_cast<unsigned>(lines),
                     static_cast<unsigned>((half + 256 * steps - 1) / (256 * steps)));
     const float s_hi = static_cast<float>(s), s_lo = static_cast<float>(s - s_hi);
+    int e;
+    const bool exact = std::frexp(s, &e) == 0.5;
     dump64_kernel<<<grid, 256, 0, stream>>>(out, out_row, src, src_row, gmap, lmap, n_map, half,
-                                            s_hi, s_lo, s);
+                                            s_hi, s_lo, s, exact);
     return cuda_check(cudaGetLastError(), "dump64_kernel launch");
 }
 

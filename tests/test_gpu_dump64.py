@@ -47,3 +47,32 @@ def test_dump_rounds_once(pkg, cuda, frames):
     off = got[ok].view(np.int32).astype(np.int64) - want[ok].view(np.int32).astype(np.int64)
     assert np.abs(off).max() <= 1 and np.count_nonzero(off) <= max(1, flat.size // 10 ** 6)
     assert np.array_equal(got[~ok & ~np.isnan(want)], want[~ok & ~np.isnan(want)])
+
+
+@pytest.mark.parametrize("frames", [1, 3, 7, 301, 1024, 4095, 1000003, 1 << 40, (1 << 40) + 1])
+def test_dump_near_ties(pkg, cuda, frames):
+    """Quotients at and within a few last places (of the double) of a tie between two
+    floats, where the 24 and 23 bits of the FP32 arithmetic do not decide: the correctly
+    rounded float of the double product, without exception."""
+    torch = cuda
+    n, nf = 3, 4096
+    s = 1.0 / frames
+    rng = np.random.default_rng(frames % 1000)
+    shape = (6, nf, 2)
+    tie = 2 * rng.integers(1 << 23, 1 << 24, size=shape).astype(np.float64) + 1
+    tie *= np.exp2(rng.integers(-24, 0, size=shape)) * rng.choice([-1.0, 1.0], size=shape)
+    v = tie / s
+    steps = rng.integers(-300, 301, size=shape)
+    steps[rng.random(shape) < 0.6] %= 4
+    v = (v.view(np.int64) + steps).view(np.float64)
+    v = np.where(np.abs(v) < 2.0 ** 65, v, 1.0)
+    eng = pkg.FxEngine(n, nf, max_frames=1, xmode=0)
+    try:
+        eng.set_accumulator(pkg.abi.CORRX_ACC_FP64)
+        out = eng.dump(torch.view_as_complex(torch.from_numpy(v).cuda().contiguous()), frames)
+        torch.cuda.synchronize()
+        got = torch.view_as_real(out).cpu().numpy()
+    finally:
+        eng.close()
+    want = (v * s).astype(np.float32)
+    assert np.count_nonzero(got.view(np.uint32) != want.view(np.uint32)) == 0
