@@ -747,16 +747,24 @@ corr_status batch_create(const std::vector<FxPlan *> &plans, const int32_t *bloc
         batch_free(b);
         return st;
     }
-    // Kernels configure themselves on first use; do that outside the capture,
-    // once for every engine a block uses.
+    // Kernels configure themselves on first use; do that outside the capture, for every
+    // engine a block uses: with its longest pass and with one frame, as the F-engine has
+    // one kernel for few transforms and one for many.
     for (int e = 0; e < n_plans && st == CORR_OK; ++e) {
-        bool used = false;
-        for (int i = 0; i < n_blocks && !used; ++i) used = plan_of(i) == plans[e];
-        if (used)
-            st = fxplan_accumulate(plans[e], d_samples, station_stride, frame_stride, d_mask,
-                                   mask_station_stride, static_cast<int>(block_first[0]), 1,
-                                   acc_of_block, b->cap, d_pmask, pmask_station_stride,
-                                   static_cast<int>(block_first[0]));
+        int longest = -1;
+        for (int i = 0; i < n_blocks; ++i)
+            if (plan_of(i) == plans[e] &&
+                (longest < 0 || block_frames[i] > block_frames[longest]))
+                longest = i;
+        if (longest < 0) continue;
+        const int first = static_cast<int>(block_first[longest]);
+        for (int frames : {1, std::min(block_frames[longest], plans[e]->max_frames)})
+            if (st == CORR_OK)
+                st = fxplan_accumulate(plans[e],
+                                       d_samples + static_cast<size_t>(first) * frame_stride,
+                                       station_stride, frame_stride, d_mask, mask_station_stride,
+                                       first, frames, acc_of_block, b->cap, d_pmask,
+                                       pmask_station_stride, first);
     }
     if (st == CORR_OK) st = cuda_check(cudaStreamSynchronize(b->cap), "warm-up");
     if (st != CORR_OK) {

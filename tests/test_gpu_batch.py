@@ -192,3 +192,38 @@ def test_packet_batch_matches_oracle(pkg, cuda, oracle, xmode):
     finally:
         lib.corrx_batch_destroy(h)
         eng.close()
+
+
+def test_batch_of_short_and_long_passes(pkg, cuda, oracle):
+    """Passes on both sides of the F-engine's choice of kernels (n_freq 8192: 1536
+    transforms) in one graph: every row equals the same block run alone."""
+    torch = cuda
+    lib = pkg.abi.load()
+    n, nf, pool = 6, 8192, 600
+    rng = np.random.default_rng(13)
+    x = rng.integers(-40, 41, size=(n, pool, 2 * nf)).astype(np.int8)
+    blocks = [(3, 40), (0, 256), (50, 300), (599, 1)]     # passes of 40, 256, 256 + 44, 1
+    first = (C.c_int64 * len(blocks))(*[b[0] for b in blocks])
+    frames = (C.c_int32 * len(blocks))(*[b[1] for b in blocks])
+    eng = pkg.FxEngine(n, nf, max_frames=256, xmode=0)
+    xs = torch.from_numpy(x).cuda()
+    rows = torch.zeros((len(blocks), n * (n + 1) // 2, nf), dtype=torch.complex64, device="cuda")
+    h = C.c_void_p()
+    assert lib.corrx_batch_create(eng.h, C.c_void_p(xs.data_ptr()), xs.stride(0), xs.stride(1),
+                                  None, 0, first, frames, len(blocks),
+                                  C.c_void_p(rows.data_ptr()), None, C.byref(h)) == 0
+    try:
+        assert lib.corrx_batch_launch(h, C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        torch.cuda.synchronize()
+        eng.check()
+        got = rows.cpu().numpy()
+        for i, (f0, nfr) in enumerate(blocks):
+            acc = eng.new_acc()
+            eng.accumulate(xs, nfr, acc, frame0=f0)
+            eng.scale(acc, nfr)
+            torch.cuda.synchronize()
+            assert np.array_equal(got[i], acc.cpu().numpy()), i
+            assert oracle.rel_rms(got[i], oracle.correlate(x[:, f0:f0 + nfr]) / nfr) < 1e-5, i
+    finally:
+        lib.corrx_batch_destroy(h)
+        eng.close()
