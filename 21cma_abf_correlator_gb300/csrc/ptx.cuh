@@ -181,16 +181,16 @@ __device__ __forceinline__ void red_add_f32x2(float2 *dst, float2 v) {
                      : "memory");
 }
 
-// dst[0..3] += {a.x, a.y, b.x, b.y} likewise; dst 16-byte aligned.
+// dst[0..3] += {a.x, a.y, b.x, b.y} likewise; dst 16-byte aligned. (One test of all four
+// values: a test and a way of its own for each pair made the tensor X-engine's launches of
+// few frames up to 5 % longer.)
 __device__ __forceinline__ void red_add_f32x4(float2 *dst, float2 a, float2 b) {
-    if ((a.x != 0.0f || a.y != 0.0f) && (b.x != 0.0f || b.y != 0.0f)) {
+    const uint32_t any = __float_as_uint(a.x) | __float_as_uint(a.y) | __float_as_uint(b.x) |
+                         __float_as_uint(b.y);
+    if ((any << 1) != 0u)   // but for the signs
         asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(gmem_addr(dst)),
                      "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y)
                      : "memory");
-    } else {
-        red_add_f32x2(dst, a);
-        red_add_f32x2(dst + 1, b);
-    }
 }
 
 // (double)x in integer arithmetic. This GPU converts (and computes) doubles at
