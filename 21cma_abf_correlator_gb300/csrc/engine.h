@@ -230,7 +230,8 @@ corr_status synth_fill_launch(int8_t *x, size_t n, uint32_t seed, cudaStream_t s
 /// Is (ct channels per tile, kt frames per stage) a feasible tensor X-engine
 /// tile for n_station inputs (TMEM columns, shared memory)?
 bool xengine_tc_shape_ok(int n_station, bool split, int ct, int kt);
-/// The widest feasible tile with 16-frame stages (*ct = 0: none).
+/// The tile of an engine that is not tuned (*ct = 0: none): the widest with 32-frame
+/// stages, but for a load ring of more than two stages.
 void xengine_tc_default_shape(int n_station, bool split, int *ct, int *kt);
 corr_status xengine_tc_launch(const XengineArgs &a, bool split, int ct, int kt, int num_sms,
                               cudaStream_t stream);

@@ -28,8 +28,9 @@
 //   28672 1525 / 2057 / 2031 -> 1132 / 1563 / 1553 us
 //   30720 2303 / 2642 / 2608 -> 1279 / 1617 / 1663 us
 //   32768 1308 / 1666 / 1675 -> 1055 / 1596 / 1570 us
-// (four frames of 18432: 16.5 -> 18.1 us.) The 8-byte formats are bound by their
-// stores: even and odd bins share 32-byte sectors and are written a transform apart.
+// (four frames of 18432: 16.5 -> 18.1 us.) Even and odd bins share 32-byte sectors and are
+// written a transform apart, which costs DRAM 1.37 times the reads (FP16 output; ncu, 256
+// frames of 32768) and the 8-byte formats most.
 // Keeping the even ones in L2 until then took 32768 hi-lo from 1712 to 1565-1596 us;
 // letting the odd ones go first 1642, and either for FP16 up to 9 % slower.
 

@@ -24,16 +24,16 @@
 // TMA ring runs on through their tiles, so that the end of one (two shuffles per
 // value, then reductions at L2) overlaps the loads of the next.
 //
-// Bound by FP32 issue: about 90 of the 128 lanes per SM and cycle in the loop
-// itself; the rest goes to scheduler imbalance (10 tiles on 4 schedulers at 24
-// inputs), stage boundaries and the last wave. Measured on one GB300, complex128
-// rows, before (4 x 4 tiles, 32 channels, cp.async, a CTA barrier per 2 to 12
+// Bound by issue: at 24 inputs (10 tiles on 4 schedulers) and 256 frames a launch, ncu has
+// 66 % of the issue slots and 52 % of the FP32 pipe busy and DRAM at 43 %; the rest goes
+// to scheduler imbalance, waits for stages and the ends of tiles. Measured on one GB300,
+// complex64 rows, before (4 x 4 tiles, 32 channels, cp.async, a CTA barrier per 2 to 12
 // frames) -> now:
-//   24 inputs, n_freq 16384, 1024 frames  1.90 -> 0.99 ms
-//   40 inputs, n_freq 16384,  512 frames  2.31 -> 1.48 ms
-//   64 inputs, n_freq  4096,  512 frames  1.94 -> 1.11 ms
-//   15 inputs, n_freq 12288,  301 frames  0.232 -> 0.135 ms
-//    4 inputs, n_freq  2048,  300 frames  0.093 -> 0.017 ms (64 one-warp CTAs before)
+//   24 inputs, n_freq 16384, 1024 frames  1.88 -> 0.95 ms
+//   40 inputs, n_freq  4096,  300 frames  0.392 -> 0.286 ms
+//   15 inputs, n_freq 12288,  301 frames  0.228 -> 0.121 ms
+//    4 inputs, n_freq 32768,   64 frames  25.4 -> 24.3 us
+//    4 inputs, n_freq  2048,  300 frames  89.6 -> 8.1 us
 
 #include <algorithm>
 #include <cmath>

@@ -92,7 +92,8 @@ corr_status corrx_scale(void *eng, void *d_acc, uint64_t frames, void *stream);
  * (corr-cuda/src/kernels.cu:252-264 accumulates complex64 across chunks).
  * CORRX_ACC_FP64: d_acc holds complex128 (16 bytes per visibility), so a row
  * summed over many launches keeps the precision of one launch; corrx_dump
- * turns it into complex64. Applies to every later corrx_accumulate*,
+ * turns it into complex64. A complex64 value that is added to counts as zero if
+ * it is subnormal. Applies to every later corrx_accumulate*,
  * corrx_run_xengine, corrx_scale and batch created from the engine. The ABI
  * contexts of corr_cuda.h always integrate in complex128 and hand back
  * complex64 rows.
@@ -154,20 +155,23 @@ corr_status corrx_check(void *eng);
  * stage is one contiguous block). xct and xkt are the tensor X-engine's
  * channels per CTA tile (2, 4, 8) and frames per pipeline stage (16, 32, 64);
  * the plain X-engine ignores them. corrx_create picks contiguous rows and the
- * widest feasible tensor tile with 32-frame stages (16 if none fits).
+ * widest feasible tensor tile with 32-frame stages (16 if none fits); where that
+ * leaves a load ring of two stages (the split form at 14-19, 30-32 and 53-63
+ * inputs) the next narrower one with 32-byte pieces, or 16-frame stages.
  */
 typedef struct corrx_tiles {
     uint32_t struct_size; /* sizeof(corrx_tiles)                                   */
     int32_t  ytile;
     int32_t  xct;
     int32_t  xkt;
-    int32_t  fplan;       /* F-engine FFT plan: 0 (three passes; four at the
-                             lengths that are not powers of two), or at n_freq
-                             16384 also 1 (four passes, twice the threads) and,
-                             with FP16 spectra (CORR_X_TC_FP16) only, 2 (the
-                             DFT stages as tcgen05 matrix products; faster, with
-                             about 1.5x the FP16 path's error; set explicitly,
-                             corrx_autotune keeps to plans 0 and 1)              */
+    int32_t  fplan;       /* F-engine FFT plan: 0 (three passes on the CUDA
+                             cores; four at 6144 with few transforms), or at
+                             n_freq 16384 also 1 (four passes, twice the
+                             threads) and, with FP16 spectra (CORR_X_TC_FP16)
+                             only, 2 (the DFT stages as tcgen05 matrix products;
+                             slower than plan 0, with about 1.5x the FP16 path's
+                             error; set explicitly, corrx_autotune keeps to
+                             plans 0 and 1)                                      */
     float    ms_fengine;  /* corrx_autotune: F-engine ms per max_frames pass       */
     float    ms_xengine;  /* corrx_autotune: X-engine ms per max_frames pass       */
 } corrx_tiles;
